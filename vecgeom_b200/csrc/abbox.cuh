@@ -255,7 +255,7 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
 
   // Steps 2 and 3 above: updates step (entering with the mother's) and hit
   // (the daughter position, -1 for the mother).  buf holds cap + 16 entries.
-  static VGB_HD void walk(const NavGeom &G, const int32_t *dl, const float4 *boxes, int nd,
+  static VGB_HD void walk(const NavGeom &G, int32_t dfirst, const float4 *boxes, int nd,
                           const V3<R> &lp, const V3<R> &ld, R &step, int &hit, AbCand *buf,
                           int cap) {
     const AbRay ray = ab_ray(lp, ld);
@@ -276,7 +276,7 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
     }
     if (m == 0) return;
     if (m > cap) {
-      walk_one_by_one(G, dl, boxes, nd, lp, ld, ray, step, hit);
+      walk_one_by_one(G, dfirst, boxes, nd, lp, ld, ray, step, hit);
       return;
     }
     L::sync();
@@ -304,13 +304,9 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
       R v = inf;  // what the candidate offers; +inf and NaN never improve
       bool inside = false;
       if (valid && !(t < b)) {
-        const int32_t pv = dl[c.d];
-        if (b < 0.) {
-          V3<R> loc;
-          inside = S::contains(G, pv, lp, loc);
-        }
+        if (b < 0.) inside = S::contains(G, dfirst + c.d, lp);
         if (!inside) {
-          const R dd = S::distance_to_in(G, pv, lp, ld, t);
+          const R dd = S::distance_to_in(G, dfirst + c.d, lp, ld, t);
           if (dd == dd) v = dd;
         }
       }
@@ -349,7 +345,7 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
 
   // The same walk for lists longer than the buffer: the next candidate is the
   // smallest (b, index) above the last one among the hits the step can reach.
-  static VGB_HD_NOINLINE void walk_one_by_one(const NavGeom &G, const int32_t *dl,
+  static VGB_HD_NOINLINE void walk_one_by_one(const NavGeom &G, int32_t dfirst,
                                               const float4 *boxes, int nd, const V3<R> &lp,
                                               const V3<R> &ld, const AbRay &ray, R &step,
                                               int &hit) {
@@ -370,16 +366,12 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
         if (ab_less(oc, best)) best = oc;
       }
       if (best.d == 0x7fffffff) break;
-      const int32_t pv = dl[best.d];
-      if (best.b < 0.f) {
-        V3<R> loc;
-        if (S::contains(G, pv, lp, loc)) {
-          t = 0.;
-          h = best.d;
-          break;
-        }
+      if (best.b < 0.f && S::contains(G, dfirst + best.d, lp)) {
+        t = 0.;
+        h = best.d;
+        break;
       }
-      const R dd = S::distance_to_in(G, pv, lp, ld, t);
+      const R dd = S::distance_to_in(G, dfirst + best.d, lp, ld, t);
       if (dd < t) {
         t = dd;
         h = best.d;
@@ -395,13 +387,12 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
   static VGB_HD bool step(const NavGeom &G, const NavPath &cur, NavPath &next, const V3<R> &lp,
                           const V3<R> &ld, R pstep, R &step_out, AbCand *buf, int cap) {
     const int32_t cv = cur.top();
-    R step = S::distance_to_out(G, cv, lp, ld, pstep);
+    const NavVol lr = nav_vol(G, cv);
+    R step = S::distance_to_out(G, lr, lp, ld, pstep);
     if (step < 0.) step = Lim<R>::inf();
-    const LogicalRec &lr = G.logicals[G.placed[cv].logical];
     const int32_t nd = lr.dcount;
-    const int32_t *dl = G.daughters + lr.dfirst;
     int hit = -1;
-    if (nd > 0) walk(G, dl, G.ab_slot + 2 * (int64_t)lr.dfirst, nd, lp, ld, step, hit, buf, cap);
+    if (nd > 0) walk(G, lr.dfirst, G.ab_slot + 2 * (int64_t)lr.dfirst, nd, lp, ld, step, hit, buf, cap);
 
     next = cur;
     if (step > pstep) {
@@ -421,11 +412,11 @@ template <class L, uint32_t kMask> struct ABBoxNavigator {
     V3<R> np = {ld.x * s6, ld.y * s6, ld.z * s6};
     np = {np.x + lp.x, np.y + lp.y, np.z + lp.z};
     if (hit != -1) {
-      const int32_t nv = dl[hit];
+      const int32_t nv = nav_placed(G, lr.dfirst + hit);
       if (next.level >= kNavMaxLevels) return false;
       next.push(nv);
       return Base::template descend<true>(G, next, nv,
-                                          nav_generic_point(G.raw[G.placed[nv].raw_xform], np), -1);
+                                          nav_generic_point(G.raw[nav_vol(G, nv).raw_xform], np), -1);
     }
     const bool ok = Base::relocate_from_path(G, next, np);
     // leaving: pop while the relocation ends in the volume being left (:390-410)

@@ -4,6 +4,7 @@
 // Host code here is compiled with -ffp-contract=off: the derived parameters of
 // each shape are computed with the same formulas and rounding as the reference
 // constructors, so the device kernels see bit-identical constants.
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -166,6 +167,7 @@ vgb_status vgb_geometry_destroy(vgb_geometry *g) {
     cudaFree(g->dev.pl_box);
     cudaFree(g->dev.ab_box);
     cudaFree(g->dev.ab_slot);
+    cudaFree(g->dev.nav_tables);
     cudaFree(g->dev.placed);
     cudaFree(g->dev.logicals);
     cudaFree(g->dev.daughters);
@@ -232,7 +234,8 @@ vgb_status vgb_logical_volume(vgb_geometry *g, const char *label, int32_t unplac
   l.unplaced = unplaced;
   l.dfirst = 0;
   l.dcount = 0;
-  l.pad = 0;
+  l.wide = l.grid = 0;
+  for (int32_t &v : l.pad) v = 0;
   g->logicals.push_back(l);
   g->logical_daughters.emplace_back();
   g->labels.push_back(label ? label : "");
@@ -282,6 +285,179 @@ vgb_status vgb_set_world(vgb_geometry *g, int32_t placed) {
 }
 
 }  // extern "C"
+
+// ---------------------------------------------------------------------------
+// boxes of the daughters, and cells over those of wide volumes (navigation.cuh)
+// ---------------------------------------------------------------------------
+namespace vgb {
+namespace {
+
+// Whether a shape's answers are bounded by its box: Contains, and every finite
+// DistanceToIn that can be the nearest, is answered by a point of the shape within
+// its tolerance.
+//   box   hits are points of a face; a point within the tolerance of a face's
+//         plane may answer a hit behind it, so boxes are tested along the whole
+//         line;
+//   tube, trd, cone, sphere, orb, polycone  hits lie at or ahead of the point, within
+//         the z planes and the radii (or on the faces); the formulas take the
+//         direction as a unit vector, which the caller checks;
+//   polyhedron  the same, or the step limit, which is never nearer than the mother's
+//         boundary;
+//   subtraction  points of the left component, or on the right one's surface inside
+//         the left one.
+// The torus moves directions as points, so its hits do not lie on the ray; the other
+// shapes are not argued here.
+bool bounded_shape(int type, const double *rec) {
+  switch (type) {
+    case VGB_SHAPE_BOX:
+    case VGB_SHAPE_TUBE:
+    case VGB_SHAPE_TRD:
+    case VGB_SHAPE_CONE:
+    case VGB_SHAPE_SPHERE:
+    case VGB_SHAPE_ORB:
+    case VGB_SHAPE_POLYCONE:
+    case VGB_SHAPE_POLYHEDRON:
+      return true;
+    case VGB_SHAPE_BOOLEAN: {
+      const BooleanP &b = *reinterpret_cast<const BooleanP *>(rec);
+      return b.op == VGB_BOOL_SUBTRACTION && b.left.type != VGB_SHAPE_BOOLEAN &&
+             b.left.type != VGB_SHAPE_POLYHEDRON && bounded_shape(b.left.type, nullptr);
+    }
+    default:
+      return false;
+  }
+}
+
+// Whether each placed volume's box may stand for it among its mother's daughters: its
+// shape is bounded and its placement a rigid motion, so that the box can be moved to
+// the mother's frame.
+void mark_bounded(vgb_geometry *g) {
+  std::vector<uint8_t> shape(g->unplaced.size()), rigid(g->raw_xforms.size());
+  for (size_t u = 0; u < shape.size(); ++u)
+    shape[u] = bounded_shape(g->unplaced[u].type, g->params.data() + g->unplaced[u].param_off);
+  for (size_t i = 0; i < rigid.size(); ++i) {
+    const double *r = g->raw_xforms[i].r;
+    bool ok = true;
+    for (int a = 0; a < 3; ++a)
+      for (int b = a; b < 3; ++b)
+        ok &= std::fabs(r[a] * r[b] + r[3 + a] * r[3 + b] + r[6 + a] * r[6 + b] -
+                        (a == b ? 1. : 0.)) < 1e-8;
+    rigid[i] = ok;
+  }
+  g->bounded.resize(g->placed.size());
+  for (size_t pv = 0; pv < g->placed.size(); ++pv) {
+    const PlacedRec &p = g->placed[pv];
+    bool ok = shape[p.unplaced] && rigid[p.raw_xform] && !(g->xforms[p.xform].flags & kXfQuirk16A);
+    for (int k = 0; ok && k < 6; ++k) ok = std::fabs(g->pl_box[6 * pv + k]) < 1e30f;
+    g->bounded[pv] = ok;
+  }
+}
+
+struct BoxItem {
+  float lo[3], hi[3];
+  int32_t d;
+};
+
+// The cell grid over a volume's daughters: cells of half the daughters' mean box
+// size, at most 64 along an axis.  A point's cell and a box's cells come from the
+// same float expression, which is monotone, so a box's range holds the cell of
+// every point of the box.
+int32_t build_grid(vgb_geometry *g, const std::vector<BoxItem> &it) {
+  CellGrid c = {};
+  float hi[3];
+  for (int k = 0; k < 3; ++k) {
+    c.org[k] = 3e38f;
+    hi[k] = -3e38f;
+    double size = 0.;
+    for (const BoxItem &b : it) {
+      c.org[k] = std::min(c.org[k], b.lo[k]);
+      hi[k] = std::max(hi[k], b.hi[k]);
+      size += (double)b.hi[k] - b.lo[k];
+    }
+    const double extent = (double)hi[k] - c.org[k];
+    const double cells = std::ceil(extent / (0.5 * size / it.size()));
+    c.n[k] = (int32_t)std::min(64., std::max(1., cells));
+    c.inv[k] = (float)(c.n[k] / (extent * (1. + 1e-5)));  // the last box ends inside the grid
+  }
+  c.first = (int32_t)g->cell_start.size();
+  // counted first, then filled in daughter order
+  const size_t ncell = (size_t)c.n[0] * c.n[1] * c.n[2];
+  auto each_cell = [&](const BoxItem &b, auto f) {
+    int a[3], z[3];
+    for (int k = 0; k < 3; ++k) {
+      a[k] = cell_of(c, k, b.lo[k]);
+      z[k] = std::min(cell_of(c, k, b.hi[k]), c.n[k] - 1);
+    }
+    for (int iz = a[2]; iz <= z[2]; ++iz)
+      for (int iy = a[1]; iy <= z[1]; ++iy)
+        for (int ix = a[0]; ix <= z[0]; ++ix) f(((size_t)iz * c.n[1] + iy) * c.n[0] + ix);
+  };
+  std::vector<int32_t> at(ncell + 1, 0);
+  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { ++at[k + 1]; });
+  at[0] = (int32_t)g->cell_items.size();
+  for (size_t k = 0; k < ncell; ++k) at[k + 1] += at[k];
+  g->cell_start.insert(g->cell_start.end(), at.begin(), at.end());
+  g->cell_items.resize(at[ncell]);
+  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { g->cell_items[at[k]++] = b.d; });
+  g->grids.push_back(c);
+  return (int32_t)g->grids.size();
+}
+
+void build_wide(vgb_geometry *g) {
+  g->grids.clear();
+  g->cell_start.clear();
+  g->cell_items.clear();
+  std::vector<BoxItem> it;
+  for (LogicalRec &l : g->logicals) {
+    l.wide = l.grid = 0;
+    if (l.dcount <= kWideDaughters) continue;
+    it.resize(l.dcount);
+    bool all = true, safety = true;
+    for (int d = 0; d < l.dcount; ++d) {
+      const int32_t pv = g->daughters[l.dfirst + d];
+      const int type = g->unplaced[g->placed[pv].unplaced].type;
+      all &= g->bounded[pv] != 0;
+      // a box's or a tube's SafetyToIn is at least its largest excess over an axis
+      // (or the radius), and so at least the distance to its box over sqrt(3); the
+      // other shapes' safeties are not argued to have such a bound
+      safety &= g->bounded[pv] && (type == VGB_SHAPE_BOX || type == VGB_SHAPE_TUBE);
+      it[d].d = d;
+      for (int k = 0; k < 3; ++k) {
+        it[d].lo[k] = g->pl_box[6 * (size_t)pv + k];
+        it[d].hi[k] = g->pl_box[6 * (size_t)pv + 3 + k];
+      }
+    }
+    l.wide = kWide | (safety ? kWideSafety : 0);
+    if (all) l.grid = build_grid(g, it);
+  }
+}
+
+// The navigator's records, from the tables already on the device.
+__global__ void k_nav_records(const PlacedRec *placed, const UnplacedRec *unplaced,
+                              const LogicalRec *logicals, const DXform *xforms,
+                              const int32_t *daughters, const float *pl_box,
+                              const uint8_t *bounded, int32_t nplaced, int32_t nslots, NavVol *vols,
+                              NavSlot *slots, float4 *slot_box) {
+  const int32_t stride = gridDim.x * blockDim.x;
+  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nplaced; k += stride) {
+    const PlacedRec p = placed[k];
+    const UnplacedRec u = unplaced[p.unplaced];
+    const LogicalRec l = logicals[p.logical];
+    vols[k] = NavVol{u.type, u.param_off, l.dfirst, l.dcount, l.wide, l.grid, p.raw_xform, p.xform};
+  }
+  for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nslots; k += stride) {
+    const int32_t pv = daughters[k];
+    const PlacedRec p = placed[pv];
+    const UnplacedRec u = unplaced[p.unplaced];
+    slots[k] = NavSlot{xforms[p.xform], u.type, u.param_off, pv, 0};
+    const SlotBox b = slot_box_of(pl_box + 6 * (int64_t)pv, bounded[pv] != 0);
+    slot_box[2 * k] = b.lo;
+    slot_box[2 * k + 1] = b.hi;
+  }
+}
+
+}  // namespace
+}  // namespace vgb
 
 vgb_status vgb::prepare_tables(vgb_geometry *g) {
   // CSR of daughters in insertion order (source/LogicalVolume.cpp:84-102)
@@ -415,6 +591,8 @@ vgb_status vgb::prepare_tables(vgb_geometry *g) {
     g->ab_slot[2 * k] = float4{b[0], b[1], b[2], 0.f};
     g->ab_slot[2 * k + 1] = float4{b[3], b[4], b[5], 0.f};
   }
+  mark_bounded(g);
+  build_wide(g);
   return VGB_OK;
 }
 
@@ -455,6 +633,52 @@ vgb_status vgb_geometry_close(vgb_geometry *g) {
   if ((s = upload(g->pl_box, &g->dev.pl_box, &g->dev.bytes)) != VGB_OK) return s;
   if ((s = upload(g->ab_box, &g->dev.ab_box, &g->dev.bytes)) != VGB_OK) return s;
   if ((s = upload(g->ab_slot, &g->dev.ab_slot, &g->dev.bytes)) != VGB_OK) return s;
+  {
+    // the navigator's tables, one allocation: what the host made in one copy, then
+    // the records a kernel makes from the tables above
+    std::vector<char> host;
+    auto put = [&](const auto &v) {
+      const size_t off = host.size(), bytes = v.size() * sizeof(v[0]);
+      host.resize((off + bytes + 255) / 256 * 256);
+      if (bytes) std::memcpy(host.data() + off, v.data(), bytes);
+      return off;
+    };
+    const size_t o_bounded = put(g->bounded), o_grids = put(g->grids),
+                 o_start = put(g->cell_start), o_items = put(g->cell_items);
+    size_t bytes = host.size();
+    auto room = [&](size_t n) {
+      const size_t off = bytes;
+      bytes += (n + 255) / 256 * 256;
+      return off;
+    };
+    const size_t np = g->placed.size(), ns = g->daughters.size();
+    const size_t o_vols = room(np * sizeof(NavVol)), o_slots = room(ns * sizeof(NavSlot)),
+                 o_box = room(2 * ns * sizeof(float4));
+    e = cudaMalloc((void **)&g->dev.nav_tables, bytes > 0 ? bytes : 1);
+    if (e != cudaSuccess) return cuda_error(e, "vgb_geometry_close: cudaMalloc");
+    g->dev.bytes += (int64_t)bytes;
+    char *base = g->dev.nav_tables;
+    if (!host.empty()) {
+      e = cudaMemcpy(base, host.data(), host.size(), cudaMemcpyHostToDevice);
+      if (e != cudaSuccess) return cuda_error(e, "vgb_geometry_close: cudaMemcpy");
+    }
+    g->dev.grids = reinterpret_cast<CellGrid *>(base + o_grids);
+    g->dev.cell_start = reinterpret_cast<int32_t *>(base + o_start);
+    g->dev.cell_items = reinterpret_cast<int32_t *>(base + o_items);
+    g->dev.vols = reinterpret_cast<NavVol *>(base + o_vols);
+    g->dev.slots = reinterpret_cast<NavSlot *>(base + o_slots);
+    g->dev.slot_box = reinterpret_cast<float4 *>(base + o_box);
+    if (np > 0) {
+      const int grid = (int)std::min<size_t>((std::max(np, ns) + 255) / 256, 148 * 8);
+      k_nav_records<<<grid, 256>>>(g->dev.placed, g->dev.unplaced, g->dev.logicals, g->dev.xforms,
+                                   g->dev.daughters, g->dev.pl_box,
+                                   reinterpret_cast<uint8_t *>(base + o_bounded), (int32_t)np,
+                                   (int32_t)ns, g->dev.vols, g->dev.slots, g->dev.slot_box);
+      e = cudaGetLastError();
+      if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+      if (e != cudaSuccess) return cuda_error(e, "vgb_geometry_close: navigation records");
+    }
+  }
   g->closed = true;
   return VGB_OK;
 }

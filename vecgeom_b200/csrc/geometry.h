@@ -41,8 +41,33 @@ struct LogicalRec {
   int32_t unplaced;
   int32_t dfirst;
   int32_t dcount;
-  int32_t pad;
+  int32_t wide;  // kWide* flags of a volume with many daughters
+  int32_t grid;  // 0: no cell grid; else its index + 1
+  int32_t pad[3];
 };
+
+// A volume with more than kWideDaughters daughters is searched through their boxes
+// (navigation.cuh).  The lists below that are scanned; in the layered detector (4
+// daughters a module, 10 in the world, 64 to 496 in a layer) only the layers are wide.
+constexpr int kWideDaughters = 32;
+enum : int32_t {
+  kWide = 1,
+  kWideSafety = 2,  // a daughter's safety is bounded by the distance to its box
+};
+
+// A grid of equal cells over a volume's daughters: cell c lists, in ascending
+// order, the positions of the daughters whose box meets it (items[start[first + c]
+// .. start[first + c + 1])).  Cells are numbered x fastest.
+struct CellGrid {
+  float org[3];    // lower corner
+  float inv[3];    // cells per mm
+  int32_t n[3];    // cells per axis
+  int32_t first;   // of the grid's cells in the start table
+  int32_t pad[2];
+};
+VGB_HD int cell_of(const CellGrid &c, int k, float v) {
+  return (int)floorf((v - c.org[k]) * c.inv[k]);
+}
 
 struct RawXform {
   double t[3];
@@ -62,6 +87,34 @@ struct NavXform {
   uint32_t pad;
 };
 
+// What the navigator reads of a placed volume, in one record (the tables above
+// reached through it take three dependent loads).
+struct alignas(16) NavVol {
+  int32_t type, param_off;  // of its shape
+  int32_t dfirst, dcount;   // of its logical volume
+  int32_t wide, grid;
+  int32_t raw_xform, xform;
+};
+static_assert(sizeof(NavVol) == 32, "read as two 16-byte words");
+// A daughter slot: the daughter's placement transform, shape and placed id.
+struct alignas(16) NavSlot {
+  DXform xf;
+  int32_t type, param_off;
+  int32_t placed;
+  int32_t pad;
+};
+static_assert(sizeof(NavSlot) == 128, "one cache line a slot");
+
+// The box of a daughter as the navigator tests it (lower and upper corner, mother's
+// frame): pl_box, or unbounded where that may not stand for the daughter.
+struct SlotBox {
+  float4 lo, hi;
+};
+VGB_HD SlotBox slot_box_of(const float *b, bool bounded) {
+  if (!bounded) return {float4{-3e38f, -3e38f, -3e38f, 0.f}, float4{3e38f, 3e38f, 3e38f, 0.f}};
+  return {float4{b[0], b[1], b[2], 0.f}, float4{b[3], b[4], b[5], 0.f}};
+}
+
 struct DeviceImage {
   double *params = nullptr;
   UnplacedRec *unplaced = nullptr;
@@ -74,6 +127,13 @@ struct DeviceImage {
   float *pl_box = nullptr;        // per placed: enclosing box in the mother's frame
   float *ab_box = nullptr;        // per placed: ABBoxManager's aligned box (float), mother frame
   float4 *ab_slot = nullptr;      // per daughter slot (CSR order): the same box as 2 float4
+  char *nav_tables = nullptr;     // the allocation that holds the tables below
+  NavVol *vols = nullptr;         // per placed volume
+  NavSlot *slots = nullptr;       // per daughter slot
+  float4 *slot_box = nullptr;     // per daughter slot: enclosing box (lower, upper), see below
+  CellGrid *grids = nullptr;      // cell grids of wide volumes, their cells and lists
+  int32_t *cell_start = nullptr;
+  int32_t *cell_items = nullptr;
   int64_t bytes = 0;
 };
 
@@ -102,6 +162,9 @@ struct vgb_geometry {
   std::vector<double> ab_box_d;        // per placed: ABBoxManager::ComputeABBox (lower, upper)
   std::vector<float> ab_box;           // the same boxes rounded to float, as navigated
   std::vector<float4> ab_slot;         // per daughter slot: (lower, 0), (upper, 0)
+  std::vector<uint8_t> bounded;        // per placed volume: its box may stand for it
+  std::vector<vgb::CellGrid> grids;    // cell grids (LogicalRec::grid)
+  std::vector<int32_t> cell_start, cell_items;
   bool abbox_ok = true;                // every placed volume's shape has an Extent
   uint32_t type_mask = 0;              // bit t set when a shape of type t exists
   int32_t world = -1;

@@ -25,7 +25,7 @@
 #include <map>
 #include <vector>
 
-#include "navigation.cuh"
+#include "nav_engine.cuh"
 
 using namespace vgb;
 
@@ -130,9 +130,8 @@ __global__ void __launch_bounds__(kSrvBlock)
       const DXform m = nav_top_matrix(G, cur);
       const V3<double> lp = xf_point(m, p);
       const V3<double> ld = xf_dir(m, d);
-      const double sf = Nav::safety(G, cur, lp);
-      double st = 0.;
-      ok = Nav::step(G, cur, nxt, lp, ld, pstep, st);
+      double sf = 0., st = 0.;
+      ok = Nav::safety_and_step(G, cur, nxt, lp, ld, pstep, sf, st);
       if (!ok) break;
       const int32_t id = nxt.top();
       h = fnv_bytes(h, &id, 4);
@@ -155,6 +154,66 @@ __global__ void __launch_bounds__(kSrvBlock)
       if (!fin) atomicAdd(live + t / kChunk, 1);
     }
   }
+}
+
+// The same step launch with a thread per track (nav_engine.cuh).
+template <uint32_t kMask> struct SrvClient {
+  const int32_t *chunks;
+  Slots S;
+  double pstep;
+  int32_t max_steps, steps_per_launch;
+  int32_t *live;
+  uint32_t *flags;
+  int32_t max_depth;
+  VGB_D void put(int64_t i, const NavTrack &t, bool ok) const {
+    const int64_t s = slot_of(chunks, i);
+    const bool fin = !ok || t.path.level == 0 || t.k >= max_steps;
+    if (!ok) atomicOr(flags, (uint32_t)VGB_NAV_ERR_DEPTH);
+    nav_store(t.path, NavStateRef{S.states + s * S.stride}, max_depth);
+    S.x[s] = t.p.x;
+    S.y[s] = t.p.y;
+    S.z[s] = t.p.z;
+    S.nsteps[s] = ok ? t.k : -1;
+    S.hash[s] = t.hash;
+    S.done[s] = fin ? 1 : 0;
+    if (!fin) atomicAdd(live + i / kChunk, 1);
+  }
+  VGB_D bool load(int64_t i, NavTrack &t) const {
+    const int64_t s = slot_of(chunks, i);
+    if (S.done[s]) return false;
+    nav_load(t.path, NavStateRef{S.states + s * S.stride});
+    t.p = {S.x[s], S.y[s], S.z[s]};
+    t.d = {S.dx[s], S.dy[s], S.dz[s]};
+    t.k = S.nsteps[s];
+    t.left = steps_per_launch;
+    t.hash = S.hash[s];
+    if (t.path.level > 0 && t.k < max_steps) return true;
+    put(i, t, true);
+    return false;
+  }
+  template <class L> VGB_D bool step(const NavGeom &G, int64_t i, NavTrack &t) const {
+    const DXform m = nav_top_matrix(G, t.path);
+    const V3<double> lp = xf_point(m, t.p), ld = xf_dir(m, t.d);
+    double sf = 0., st = 0.;
+    const bool ok =
+        Navigator<L, kMask>::safety_and_step(G, t.path, t.path, lp, ld, pstep, sf, st);
+    if (ok) {
+      const int32_t id = t.path.top();
+      t.hash = fnv_bytes(t.hash, &id, 4);
+      t.hash = fnv_bytes(t.hash, &st, 8);
+      t.hash = fnv_bytes(t.hash, &sf, 8);
+      t.p = {t.p.x + t.d.x * st, t.p.y + t.d.y * st, t.p.z + t.d.z * st};
+      ++t.k;
+      if (--t.left > 0 && t.path.level > 0 && t.k < max_steps) return true;
+    }
+    if (L::lane() == 0) put(i, t, ok);
+    return false;
+  }
+};
+template <uint32_t kMask>
+__global__ void __launch_bounds__(kEngThreads, kEngBlocks)
+    k_srv_step_tracks(const NavGeom G, const SrvClient<kMask> client, int64_t ntracks) {
+  nav_engine(G, client, ntracks);
 }
 
 // results of the listed chunks' slots, in chunk-list order
@@ -180,6 +239,12 @@ NavGeom server_geom(const vgb_geometry *g) {
   G.ab_slot = g->dev.ab_slot;
   G.world = g->world;
   G.max_depth = g->max_depth;
+  G.vols = g->dev.vols;
+  G.slots = g->dev.slots;
+  G.slot_box = g->dev.slot_box;
+  G.grids = g->dev.grids;
+  G.cell_start = g->dev.cell_start;
+  G.cell_items = g->dev.cell_items;
   return G;
 }
 
@@ -262,7 +327,11 @@ template <uint32_t kMask> void launch_admit(vgb_server *s, int64_t nt) {
       server_geom(s->g), s->d_chunks, nt, s->d_in, s->d_valid, s->S, s->g->dev.nav_flags);
 }
 template <uint32_t kMask> void launch_step(vgb_server *s, int64_t nt) {
-  if (s->screen)
+  if (nav_by_threads<kMask>(NavCall::kTrace, nt)) {
+    const SrvClient<kMask> c = {s->d_chunks, s->S,       s->pstep,          s->max_steps,
+                                s->steps_per_launch, s->d_live, s->g->dev.nav_flags, s->g->max_depth};
+    k_srv_step_tracks<kMask><<<engine_grid(nt), kEngThreads, 0, s->stream>>>(server_geom(s->g), c, nt);
+  } else if (s->screen)
     k_srv_step<kMask, true><<<srv_grid(nt), kSrvBlock, 0, s->stream>>>(
         server_geom(s->g), s->d_chunks, nt, s->S, s->pstep, s->max_steps, s->steps_per_launch,
         s->d_live, s->g->dev.nav_flags);
