@@ -71,6 +71,11 @@ template <class R> struct PolyconeOps {
   struct Walk {
     int index, increment;
     R distance;
+    // DistanceToIn: what the reachability test needs of the ray, computed once: whether
+    // it applies, 1 / v.z (0: parallel to the planes) and the parameter of the ray's
+    // closest approach to the axis (0 for a ray along it)
+    bool test;
+    R invz, tclose;
     // DistanceToOut: the distance so far, the steps taken, the point in the
     // current section's frame
     int istep;
@@ -85,6 +90,15 @@ template <class R> struct PolyconeOps {
     if (w.index == -1) w.index = 0;
     if (w.index == -2) w.index = p.nsec - 1;
     w.distance = Lim<R>::inf();
+    // the cone arithmetic takes v as a unit vector (1 - v.z^2 for v.x^2 + v.y^2);
+    // for any other v (the reference's 0x16A rotation code hands one over) its
+    // answers are not points of the surface along the ray, so every section is
+    // evaluated; so it is for a point farther than 1e9
+    const R a = v.x * v.x + v.y * v.y;
+    w.test = fabs(a + v.z * v.z - (R)1) < (R)1e-10 &&
+             fabs(q.x) + fabs(q.y) + fabs(q.z) < (R)1e9;
+    w.invz = v.z != 0 ? (R)1 / v.z : (R)0;
+    w.tclose = a > 0 ? -(q.x * v.x + q.y * v.y) / a : (R)0;
     return false;
   }
   // Every finite answer of the cone's DistanceToIn is a point of the section's
@@ -96,25 +110,48 @@ template <class R> struct PolyconeOps {
   // kInfinity from the section: the walk skips that evaluation and goes on as
   // after an infinite answer.  (The same test inside the single cone's
   // DistanceToIn, which rejects such rays cheaply on its own, measured slower.)
-  static VGB_HD bool out_of_reach(const PolySec &s, const V3<R> &q, const V3<R> &v) {
-    // the cone arithmetic takes v as a unit vector (1 - v.z^2 for v.x^2 + v.y^2);
-    // for any other v (the reference's 0x16A rotation code hands one over) its
-    // answers are not points of the surface along the ray, so it is evaluated
-    if (!(fabs(v.x * v.x + v.y * v.y + v.z * v.z - (R)1) < (R)1e-10)) return false;
+  static VGB_HD bool out_of_reach(const PolySec &s, const V3<R> &q, const V3<R> &v,
+                                  const Walk &w) {
+    if (!w.test) return false;
     const R dz = (R)s.cone.dz, zc = (R)s.shift;
     const R mz = (R)1e-3 + (R)1e-6 * (fabs(zc) + dz);
+    const R zlo = zc - dz - mz, zhi = zc + dz + mz;
+    // the ray's part in the slab.  A ray within 1e-12 of parallel to the planes rises
+    // less than 1e-3 on its way to the axis (points lie within 1e9 of it): it is in
+    // the slab for good, or never.
+    R t0 = 0, t1 = Lim<R>::inf();
+    if (fabs(v.z) > (R)1e-12) {
+      const R ta = (zlo - q.z) * w.invz, tb = (zhi - q.z) * w.invz;
+      t0 = vmax(vmin(ta, tb), (R)0);
+      t1 = vmax(ta, tb);
+      if (t0 > t1) return true;  // the slab lies behind the point
+    } else if (fabs(q.z - zc) > dz + mz + (R)1e-3) {
+      return true;
+    }
     const R rmax = vmax((R)s.cone.rmax1, (R)s.cone.rmax2);
-    return ray_beyond_radius(q, v, zc - dz - mz, zc + dz + mz, rmax + (R)1e-3 + (R)1e-6 * rmax);
+    const R rb = rmax + (R)1e-3 + (R)1e-6 * rmax;
+    const R tm = vmin(vmax(w.tclose, t0), t1);
+    const R x = q.x + tm * v.x, y = q.y + tm * v.y;
+    return x * x + y * y > rb * rb;
   }
 
+  // One step: past the sections out of reach (a few operations each), then the
+  // evaluation of one section, so the lanes of a warp evaluate together whatever they
+  // skipped.
   static VGB_HD bool dti_step(const PolyconeP &p, const V3<R> &q, const V3<R> &v, R smax,
                               Walk &w) {
-    const PolySec &s = sec(p, w.index);
-    w.distance = out_of_reach(s, q, v) ? Lim<R>::inf()
-                                       : C::distance_to_in(s.cone, shifted(q, s), v, smax);
-    if (w.distance < Lim<R>::inf() || !w.increment) return true;
-    w.index += w.increment;
-    return !(w.index >= 0 && w.index < p.nsec);
+    bool over = false;
+    while (!over && out_of_reach(sec(p, w.index), q, v, w)) {
+      w.index += w.increment;
+      over = !w.increment || !(w.index >= 0 && w.index < p.nsec);
+    }
+    if (!over) {
+      const PolySec &s = sec(p, w.index);
+      w.distance = C::distance_to_in(s.cone, shifted(q, s), v, smax);
+      w.index += w.increment;
+      over = w.distance < Lim<R>::inf() || !w.increment || !(w.index >= 0 && w.index < p.nsec);
+    }
+    return over;
   }
   static VGB_HD R dti_end(const PolyconeP &, const V3<R> &, const V3<R> &, R, const Walk &w) {
     return w.distance;

@@ -40,7 +40,7 @@ struct PhSeg {
   int32_t inner_off, inner_n;
   int32_t phi_off, phi_n;
   int32_t has_inner;
-  int32_t pad;
+  float inner_r;  // no inner quadrilateral reaches farther from the z axis; 0: not known
 };
 
 struct PolyhedronP {
@@ -269,7 +269,8 @@ template <class R> struct PolyhedronOps {
   }
 
   // DistanceToInZSegment (:440-470)
-  static VGB_HD R dti_segment(const PolyhedronP &p, int zi, const V3<R> &pt, const V3<R> &dir) {
+  static VGB_HD R dti_segment(const PolyhedronP &p, int zi, const V3<R> &pt, const V3<R> &dir,
+                              R close2) {
     const PhSeg &s = seg(p, zi);
     R distance = quads_dti<false>(p, s.outer_off, s.outer_n, pt, dir);
     bool done = distance < Lim<R>::inf();
@@ -277,17 +278,18 @@ template <class R> struct PolyhedronOps {
     if (p.has_phi_cutout) distance = quads_dti<false>(p, s.phi_off, s.phi_n, pt, dir);
     done |= distance < Lim<R>::inf();
     if (done) return distance;
-    if (s.has_inner) distance = quads_dti<true>(p, s.inner_off, s.inner_n, pt, dir);
+    if (s.has_inner && !past_inner(s, close2))
+      distance = quads_dti<true>(p, s.inner_off, s.inner_n, pt, dir);
     return distance;
   }
 
   // DistanceToOutZSegment (:472-500)
   static VGB_HD R dto_segment(const PolyhedronP &p, int zi, R zMin, R zMax, const V3<R> &pt,
-                              const V3<R> &dir) {
+                              const V3<R> &dir, R close2) {
     const PhSeg &s = seg(p, zi);
     bool done = false;
     R distance = Lim<R>::inf();
-    if (s.has_inner) {
+    if (s.has_inner && !past_inner(s, close2)) {
       distance = quads_dti<false>(p, s.inner_off, s.inner_n, pt, dir);
       done = distance < Lim<R>::inf();
       if (done) return distance;
@@ -335,7 +337,21 @@ template <class R> struct PolyhedronOps {
     int zi;
     bool right;
     R distance;
+    R close2;  // squared distance of the ray's closest approach to the z axis
   };
+  static VGB_HD R closest_approach2(const V3<R> &pt, const V3<R> &dir) {
+    const R a = dir.x * dir.x + dir.y * dir.y;
+    R t = a > 0 ? -(pt.x * dir.x + pt.y * dir.y) / a : (R)0;
+    t = t > 0 ? t : (R)0;
+    const R x = pt.x + t * dir.x, y = pt.y + t * dir.y;
+    return fabs(pt.x) + fabs(pt.y) < (R)1e9 ? x * x + y * y : (R)0;
+  }
+  // An inner side is hit within the segment's inner_r of the axis; a ray that stays
+  // farther from it, by more than the rounding of either, hits none.
+  static VGB_HD bool past_inner(const PhSeg &s, R close2) {
+    const R r = (R)s.inner_r + (R)1e-3;
+    return s.inner_r > 0 && close2 > r * r;
+  }
   static VGB_HD bool dti_begin(const PolyhedronP &p, const V3<R> &pt, const V3<R> &dir, R smax,
                                Walk &w, R &res) {
     const V3<R> bp = {pt.x, pt.y, pt.z - (R)p.btube_offset};
@@ -357,11 +373,12 @@ template <class R> struct PolyhedronOps {
     w.zi = zi;
     w.right = dir.z >= 0;
     w.distance = Lim<R>::inf();
+    w.close2 = closest_approach2(pt, dir);
     return false;
   }
   static VGB_HD bool dti_step(const PolyhedronP &p, const V3<R> &pt, const V3<R> &dir, R,
                               Walk &w) {
-    w.distance = dti_segment(p, w.zi, pt, dir);
+    w.distance = dti_segment(p, w.zi, pt, dir, w.close2);
     if (w.distance >= 0 && w.distance < Lim<R>::inf()) return true;
     if (w.right) return !(++w.zi < p.nseg);
     return !(--w.zi >= 0);
@@ -388,12 +405,13 @@ template <class R> struct PolyhedronOps {
     w.zi = zi < 0 ? 0 : (zi >= zMax ? zMax - 1 : zi);
     w.right = dir.z >= 0;
     w.distance = Lim<R>::inf();
+    w.close2 = closest_approach2(pt, dir);
     return false;
   }
   static VGB_HD bool dto_step(const PolyhedronP &p, const V3<R> &pt, const V3<R> &dir, R,
                               Walk &w) {
     const int zi = w.zi;
-    w.distance = dto_segment(p, zi, zplane(p, zi), zplane(p, zi + 1), pt, dir);
+    w.distance = dto_segment(p, zi, zplane(p, zi), zplane(p, zi + 1), pt, dir, w.close2);
     if (w.distance >= 0 && w.distance < Lim<R>::inf()) return true;
     if (w.right) {
       if (zplane(p, zi) - pt.z > w.distance) return true;
@@ -467,16 +485,30 @@ template <class R> struct PolyhedronOps {
     int zi = find_z(p, pt.z);
     zi = zi < 0 ? 0 : (zi >= zMax ? zMax - 1 : zi);
     const int phiIndex = find_phi(p, pt);
-    for (int z = zi; z < zMax;) {
-      const R dz = vmax(zplane(p, z) - pt.z, pt.z - zplane(p, z + 1));
-      if (may_lower(dz, s)) s = vmin(s, seg_safety2(p, z, phiIndex, pt));
-      ++z;
-      if (zplane(p, z) - pt.z > s) break;
-    }
-    for (int z = zi - 1; z >= 0; --z) {
-      const R dz = vmax(zplane(p, z) - pt.z, pt.z - zplane(p, z + 1));
-      if (may_lower(dz, s)) s = vmin(s, seg_safety2(p, z, phiIndex, pt));
-      if (pt.z - zplane(p, z) > s) break;
+    // The walk goes up from the point's segment, then down from below it.  Each round
+    // passes the segments that cannot lower the minimum and evaluates the next one
+    // that may, so the lanes of a warp evaluate together, whichever segments they
+    // passed and whichever way they go.
+    int z = zi;
+    bool up = true;
+    auto next = [&]() {  // the segment after z, by the reference's stopping rule
+      if (up) {
+        ++z;
+        if (zplane(p, z) - pt.z > s || z >= zMax) {
+          up = false;
+          z = zi - 1;
+        }
+      } else if (pt.z - zplane(p, z) > s) {
+        z = -1;
+      } else {
+        --z;
+      }
+    };
+    for (;;) {
+      while (z >= 0 && !may_lower(vmax(zplane(p, z) - pt.z, pt.z - zplane(p, z + 1)), s)) next();
+      if (z < 0) break;
+      s = vmin(s, seg_safety2(p, z, phiIndex, pt));
+      next();
     }
     endcaps_safety2(p, pt, s);
     return sqrt(s);

@@ -615,6 +615,8 @@ std::vector<double> make_polyhedron(double phiStart, double phiDelta, int sides,
       quad_set(q, iv[vi(p, k)], iv[vi(p, k + 1)], iv[vi(p + 1, k + 1)], iv[vi(p + 1, k)]);
       if (wrong_normal(quad_normal(q), iv[vi(p, k)])) quad_flip(q);
       quads.push_back(q);
+      for (int c = 0; c < 4; ++c)
+        s.inner_r = std::max(s.inner_r, std::nextafter((float)std::hypot(q.c[c][0], q.c[c][1]), 3e38f));
     }
     s.phi_off = (int32_t)quads.size();
     s.phi_n = phi_n[p];
