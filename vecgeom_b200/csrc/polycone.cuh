@@ -93,11 +93,12 @@ template <class R> struct PolyconeOps {
     // the cone arithmetic takes v as a unit vector (1 - v.z^2 for v.x^2 + v.y^2);
     // for any other v (the reference's 0x16A rotation code hands one over) its
     // answers are not points of the surface along the ray, so every section is
-    // evaluated; so it is for a point farther than 1e9
+    // evaluated; so it is for a point that is not finite
     const R a = v.x * v.x + v.y * v.y;
     w.test = fabs(a + v.z * v.z - (R)1) < (R)1e-10 &&
-             fabs(q.x) + fabs(q.y) + fabs(q.z) < (R)1e9;
-    w.invz = v.z != 0 ? (R)1 / v.z : (R)0;
+             fabs(q.x) + fabs(q.y) + fabs(q.z) < Lim<R>::inf();
+    // a |v.z| below 1e-290 never reaches another slab: parallel to the planes
+    w.invz = fabs(v.z) > (R)1e-290 ? (R)1 / v.z : (R)0;
     w.tclose = a > 0 ? -(q.x * v.x + q.y * v.y) / a : (R)0;
     return false;
   }
@@ -116,17 +117,15 @@ template <class R> struct PolyconeOps {
     const R dz = (R)s.cone.dz, zc = (R)s.shift;
     const R mz = (R)1e-3 + (R)1e-6 * (fabs(zc) + dz);
     const R zlo = zc - dz - mz, zhi = zc + dz + mz;
-    // the ray's part in the slab.  A ray within 1e-12 of parallel to the planes rises
-    // less than 1e-3 on its way to the axis (points lie within 1e9 of it): it is in
-    // the slab for good, or never.
+    // the ray's part in the slab
     R t0 = 0, t1 = Lim<R>::inf();
-    if (fabs(v.z) > (R)1e-12) {
+    if (w.invz != 0) {
       const R ta = (zlo - q.z) * w.invz, tb = (zhi - q.z) * w.invz;
       t0 = vmax(vmin(ta, tb), (R)0);
       t1 = vmax(ta, tb);
       if (t0 > t1) return true;  // the slab lies behind the point
-    } else if (fabs(q.z - zc) > dz + mz + (R)1e-3) {
-      return true;
+    } else if (q.z < zlo || q.z > zhi) {
+      return true;  // parallel to the slab, outside it
     }
     const R rmax = vmax((R)s.cone.rmax1, (R)s.cone.rmax2);
     const R rb = rmax + (R)1e-3 + (R)1e-6 * rmax;
@@ -137,7 +136,9 @@ template <class R> struct PolyconeOps {
 
   // One step: past the sections out of reach (a few operations each), then the
   // evaluation of one section, so the lanes of a warp evaluate together whatever they
-  // skipped.
+  // skipped.  Bound by the divergence of the cone's DistanceToIn (9 of 32 lanes
+  // active); 10 planes, 2^22 mixed points: 582 us with the test's three divisions in
+  // every section's step, 441 with this one.
   static VGB_HD bool dti_step(const PolyconeP &p, const V3<R> &q, const V3<R> &v, R smax,
                               Walk &w) {
     bool over = false;

@@ -347,7 +347,11 @@ template <class R> struct PolyhedronOps {
     return fabs(pt.x) + fabs(pt.y) < (R)1e9 ? x * x + y * y : (R)0;
   }
   // An inner side is hit within the segment's inner_r of the axis; a ray that stays
-  // farther from it, by more than the rounding of either, hits none.
+  // farther from it, by more than the rounding of either, hits none.  8 sides, 5
+  // segments, rmin a quarter of rmax, 2^22 mixed points: DistanceToIn 529 -> 441 us,
+  // DistanceToOut on 2^21 279 -> 235 us.  (Steps of one quadrilateral instead of a
+  // segment's lists, to keep more than 7 of 32 lanes active: 587 and 570 us, the lists'
+  // scans diverge more than the evaluations they regroup.)
   static VGB_HD bool past_inner(const PhSeg &s, R close2) {
     const R r = (R)s.inner_r + (R)1e-3;
     return s.inner_r > 0 && close2 > r * r;
@@ -488,7 +492,8 @@ template <class R> struct PolyhedronOps {
     // The walk goes up from the point's segment, then down from below it.  Each round
     // passes the segments that cannot lower the minimum and evaluates the next one
     // that may, so the lanes of a warp evaluate together, whichever segments they
-    // passed and whichever way they go.
+    // passed and whichever way they go (2^22 points: SafetyToIn 371 -> 361 us,
+    // SafetyToOut on 2^21 177 -> 163 us).
     int z = zi;
     bool up = true;
     auto next = [&]() {  // the segment after z, by the reference's stopping rule
