@@ -146,7 +146,8 @@ template <> struct RegroupedWalk<PolyconeOps<double>, VGB_OP_DISTANCE_TO_OUT> : 
 template <> struct RegroupedWalk<PolyhedronOps<double>, VGB_OP_DISTANCE_TO_IN> : std::true_type {};
 template <> struct RegroupedWalk<PolyhedronOps<double>, VGB_OP_DISTANCE_TO_OUT> : std::true_type {};
 
-template <class Ops, class P, int OP, class IO, class PointOf>
+// kInside (DistanceToOut): only where Contains() holds; kInfinity elsewhere.
+template <class Ops, class P, int OP, bool kInside = false, class W = Ops, class IO, class PointOf>
 __device__ __forceinline__ void walk_regrouped(const P &prm, const DXform &X, const IO &io,
                                                double *out, PointOf point_of, int64_t end) {
   using R = double;
@@ -157,7 +158,7 @@ __device__ __forceinline__ void walk_regrouped(const P &prm, const DXform &X, co
   int64_t i = -1;    // the lane's point, -1: none
   V3<R> q = {0, 0, 0}, v = {0, 0, 0};
   R smax = 0;
-  typename Ops::Walk w;
+  typename W::Walk w;
   while (true) {
     const bool free_lane = i < 0;
     const unsigned m = __ballot_sync(kFull, free_lane);
@@ -172,11 +173,13 @@ __device__ __forceinline__ void walk_regrouped(const P &prm, const DXform &X, co
         if constexpr (kIn) {
           q = xf_point(X, mq);
           v = dti_dir<Ops>(X, md);
-          done = Ops::dti_begin(prm, q, v, smax, w, res);
+          done = W::dti_begin(prm, q, v, smax, w, res);
         } else {
           q = mq;
           v = md;
-          done = Ops::dto_begin(prm, q, v, smax, w, res);
+          res = Lim<R>::inf();
+          done = kInside && !Ops::contains(prm, xf_point(X, mq));
+          if (!done) done = W::dto_begin(prm, q, v, smax, w, res);
         }
         if (done)
           out[pi] = res;  // settled in the set-up; the lane stays free
@@ -190,14 +193,14 @@ __device__ __forceinline__ void walk_regrouped(const P &prm, const DXform &X, co
     if (i >= 0) {
       bool ended;
       if constexpr (kIn)
-        ended = Ops::dti_step(prm, q, v, smax, w);
+        ended = W::dti_step(prm, q, v, smax, w);
       else
-        ended = Ops::dto_step(prm, q, v, smax, w);
+        ended = W::dto_step(prm, q, v, smax, w);
       if (ended) {
         if constexpr (kIn)
-          out[i] = Ops::dti_end(prm, q, v, smax, w);
+          out[i] = W::dti_end(prm, q, v, smax, w);
         else
-          out[i] = Ops::dto_end(prm, q, v, smax, w);
+          out[i] = W::dto_end(prm, q, v, smax, w);
         i = -1;
       }
     }
@@ -269,6 +272,90 @@ __device__ __forceinline__ void fused_point(const P &prm, const DXform &X, const
     R r = Lim<R>::inf();
     if (!dto_inside || c) r = Ops::distance_to_out(prm, m, d, ldg(io.step + i));
     static_cast<double *>(io.out[VGB_OP_DISTANCE_TO_OUT])[i] = r;
+  }
+}
+
+// The fused ops of an expensive shape: one launch whose block rows (blockIdx.y) each do
+// one group of ops over all points, DistanceToIn, DistanceToOut, or the point ops
+// (Contains, Inside, the safeties), in the forms of the batch kernels (tables in shared
+// memory, regrouped walks).  One thread doing every op of its point in turn holds every
+// op's registers and walks with its warp half idle; the rows run at the same time, so a
+// small batch takes the longest row's latency instead of the sum.
+// All six ops, local ones inside only, us, one thread per point / rows: 500,009 mixed
+// points cone 40 / 31, sphere 54 / 46, torus 104 / 68, polycone 239 / 162, polyhedron
+// 381 / 260, box minus tube 83 / 53; 100,003 points polycone 75 / 51, polyhedron 93 / 66;
+// from 16,411 points down both take the launch's time.  (Three launches instead of three
+// rows: polyhedron 328 and 126.)
+// The tube and the cheaper shapes stay on k_fused: they are bound by the points' loads,
+// which the rows make three times (tube on 2^22 points 192 us; by rows 199).
+template <class P> struct SplitFused : std::false_type {};
+template <> struct SplitFused<TorusP> : std::true_type {};
+template <> struct SplitFused<PolyconeP> : std::true_type {};
+template <> struct SplitFused<PolyhedronP> : std::true_type {};
+template <> struct SplitFused<BooleanP> : std::true_type {};
+template <> struct SplitFused<ConeP> : std::true_type {};
+template <> struct SplitFused<SphereP> : std::true_type {};
+constexpr uint32_t kPointOps = (1u << VGB_OP_CONTAINS) | (1u << VGB_OP_INSIDE) |
+                               (1u << VGB_OP_SAFETY_TO_IN) | (1u << VGB_OP_SAFETY_TO_OUT);
+
+// DistanceToOut in one step, for walk_regrouped: where only the points inside count,
+// the lanes of the points outside take the next ones.
+template <class Ops> struct OneStepOut {
+  struct Walk {
+    double distance;
+  };
+  template <class P>
+  static VGB_D bool dto_begin(const P &, const V3<double> &, const V3<double> &, double, Walk &,
+                              double &) {
+    return false;
+  }
+  template <class P>
+  static VGB_D bool dto_step(const P &p, const V3<double> &q, const V3<double> &v, double smax,
+                             Walk &w) {
+    w.distance = Ops::distance_to_out(p, q, v, smax);
+    return true;
+  }
+  template <class P>
+  static VGB_D double dto_end(const P &, const V3<double> &, const V3<double> &, double,
+                              const Walk &w) {
+    return w.distance;
+  }
+};
+
+template <class Ops, class P>
+__global__ void __launch_bounds__(kBatchBlock, DistanceBlocks<Ops>::value)
+    k_fused_split(const P prm, const DXform X, const FusedIO io, int32_t stage) {
+  P sp = prm;
+  if constexpr (Stageable<P>::value) {
+    if (stage > 0) {
+      for (int k = threadIdx.x; k < stage; k += blockDim.x) vgb_stage[k] = prm.base[k];
+      __syncthreads();
+      sp.base = vgb_stage;
+    }
+  }
+  // row y is the y-th group present
+  const bool dti = io.ops & (1u << VGB_OP_DISTANCE_TO_IN);
+  const bool dto = io.ops & (1u << VGB_OP_DISTANCE_TO_OUT);
+  const int row = (int)blockIdx.y;
+  if (dti && row == 0) {
+    const BatchIO b = {io.x, io.y, io.z, io.dx, io.dy, io.dz, io.step,
+                       io.out[VGB_OP_DISTANCE_TO_IN], nullptr, io.n, 0, 0};
+    batch_loop<Ops, P, VGB_OP_DISTANCE_TO_IN>(sp, X, b);
+  } else if (dto && row == (dti ? 1 : 0)) {
+    using W = std::conditional_t<RegroupedWalk<Ops, VGB_OP_DISTANCE_TO_OUT>::value, Ops,
+                                 OneStepOut<Ops>>;
+    const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    double *out = static_cast<double *>(io.out[VGB_OP_DISTANCE_TO_OUT]);
+    auto point_of = [=](int64_t s) { return 32 * gw + 32 * nw * (s >> 5) + (s & 31); };
+    if (io.flags & (VGB_FUSED_DTO_INSIDE_ONLY | VGB_FUSED_LOCAL_INSIDE_ONLY))
+      walk_regrouped<Ops, P, VGB_OP_DISTANCE_TO_OUT, true, W>(sp, X, io, out, point_of, io.n);
+    else
+      walk_regrouped<Ops, P, VGB_OP_DISTANCE_TO_OUT, false, W>(sp, X, io, out, point_of, io.n);
+  } else {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < io.n; i += stride)
+      fused_point<Ops, P, kPointOps>(sp, X, io, i);
   }
 }
 

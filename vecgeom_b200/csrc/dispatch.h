@@ -13,4 +13,11 @@ vgb_status launch_batch_f64(const vgb_geometry *g, int32_t placed, int op, const
                             cudaStream_t s, int precision = VGB_PREC_FP64);
 vgb_status launch_fused_f64(const vgb_geometry *g, int32_t placed, const FusedIO &io,
                             cudaStream_t s);
+// one shape's launches (batch_launch.cuh)
+template <class Ops, class P> struct BatchLaunch {
+  static vgb_status batch(const P &prm, const DXform &X, int op, BatchIO io, cudaStream_t s,
+                          int32_t rec_len, int precision);
+  static vgb_status fused(const P &prm, const DXform &X, const FusedIO &io, cudaStream_t s,
+                          int32_t rec_len);
+};
 }  // namespace vgb
