@@ -244,6 +244,13 @@ vgb_status vgb_batch(const vgb_geometry *g, int32_t placed, int32_t op, int64_t 
                      const double *dy, const double *dz, const double *step_max, void *out,
                      int32_t *aux, int32_t daughter, int32_t precision, void *stream);
 
+/* vgb_batch for arrays the caller knows to be device memory: the same call without
+ * asking the driver about them. */
+vgb_status vgb_batch_device(const vgb_geometry *g, int32_t placed, int32_t op, int64_t n,
+                            const double *x, const double *y, const double *z, const double *dx,
+                            const double *dy, const double *dz, const double *step_max, void *out,
+                            int32_t *aux, int32_t daughter, int32_t precision, void *stream);
+
 /* Per-operation forms with the reference's argument order. */
 vgb_status vgb_Contains(const vgb_geometry *g, int32_t placed, int64_t n, const double *x,
                         const double *y, const double *z, uint8_t *out, void *stream);

@@ -93,6 +93,7 @@ SIGNATURES = {
     "vgb_geometry_export_cpp": (ctypes.c_int, [_vp, _vp, ctypes.c_size_t,
                                                ctypes.POINTER(ctypes.c_size_t)]),
     "vgb_batch": (ctypes.c_int, [_vp, _i32, _i32, _i64] + [_vp] * 9 + [_i32, _i32, _vp]),
+    "vgb_batch_device": (ctypes.c_int, [_vp, _i32, _i32, _i64] + [_vp] * 9 + [_i32, _i32, _vp]),
     "vgb_batch_fused": (ctypes.c_int, [_vp, _i32, _u32, _i64] + [_vp] * 8 + [_u32, _i32, _vp]),
     "vgb_Contains": (ctypes.c_int, [_vp, _i32, _i64, _vp, _vp, _vp, _vp, _vp]),
     "vgb_Inside": (ctypes.c_int, [_vp, _i32, _i64, _vp, _vp, _vp, _vp, _vp]),
@@ -155,6 +156,26 @@ def lib():
         fn.argtypes = args
     _lib = L
     return L
+
+
+_pycall = None
+
+
+def pycall():
+    """The native call module (csrc/pycall.cpp), which links to the torch libraries of
+    the running process (called with tensors in hand); raises if it was not built."""
+    global _pycall
+    if _pycall is None:
+        import importlib.util
+        path = os.path.join(_HERE, "lib", "_pycall.so")
+        if not os.path.exists(path):
+            raise ImportError(f"_pycall.so not found at {path}: build it with "
+                              "`make -C vecgeom_b200/csrc` (or __graft_entry__.build())")
+        spec = importlib.util.spec_from_file_location("_pycall", path)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+        _pycall = m
+    return _pycall
 
 
 def check(status: int) -> None:

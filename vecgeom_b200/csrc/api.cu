@@ -176,13 +176,13 @@ vgb_status staged_call(vgb_geometry *g, cudaStream_t s, int64_t n, int64_t cap,
 
 extern "C" {
 
-vgb_status vgb_batch(const vgb_geometry *gc, int32_t placed, int32_t op, int64_t n,
-                     const double *x, const double *y, const double *z, const double *dx,
-                     const double *dy, const double *dz, const double *step_max, void *out,
-                     int32_t *aux, int32_t daughter, int32_t precision, void *stream) {
+// What every batch call checks of its arguments.
+static vgb_status check_batch(const vgb_geometry *gc, int32_t placed, int32_t op, int64_t n,
+                              const double *x, const double *y, const double *z, const double *dx,
+                              const double *dy, const double *dz, const double *step_max,
+                              const void *out, const int32_t *aux, int32_t precision) {
   vgb_status st = check_geometry(gc, placed, "vgb_batch");
   if (st != VGB_OK) return st;
-  vgb_geometry *g = const_cast<vgb_geometry *>(gc);
   if (op < 0 || op >= VGB_OP_COUNT) return set_error(VGB_EINVAL, "vgb_batch: unknown op %d", op);
   if (precision != VGB_PREC_FP64 && precision != VGB_PREC_FP32_REFINE)
     return set_error(VGB_EINVAL, "vgb_batch: unknown precision %d", precision);
@@ -194,6 +194,28 @@ vgb_status vgb_batch(const vgb_geometry *gc, int32_t placed, int32_t op, int64_t
   if (op_needs_step(op) && !step_max)
     return set_error(VGB_EINVAL, "vgb_batch: op %d needs step_max", op);
   if (op_needs_aux(op) && !aux) return set_error(VGB_EINVAL, "vgb_batch: op %d needs aux", op);
+  return VGB_OK;
+}
+
+vgb_status vgb_batch_device(const vgb_geometry *g, int32_t placed, int32_t op, int64_t n,
+                            const double *x, const double *y, const double *z, const double *dx,
+                            const double *dy, const double *dz, const double *step_max, void *out,
+                            int32_t *aux, int32_t daughter, int32_t precision, void *stream) {
+  const vgb_status st =
+      check_batch(g, placed, op, n, x, y, z, dx, dy, dz, step_max, out, aux, precision);
+  if (st != VGB_OK || n == 0) return st;
+  const BatchIO io{x, y, z, dx, dy, dz, step_max, out, aux, n, daughter, 0};
+  return launch_batch_f64(g, placed, op, io, static_cast<cudaStream_t>(stream), precision);
+}
+
+vgb_status vgb_batch(const vgb_geometry *gc, int32_t placed, int32_t op, int64_t n,
+                     const double *x, const double *y, const double *z, const double *dx,
+                     const double *dy, const double *dz, const double *step_max, void *out,
+                     int32_t *aux, int32_t daughter, int32_t precision, void *stream) {
+  vgb_status st =
+      check_batch(gc, placed, op, n, x, y, z, dx, dy, dz, step_max, out, aux, precision);
+  if (st != VGB_OK || n == 0) return st;
+  vgb_geometry *g = const_cast<vgb_geometry *>(gc);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
 
   const PtrKind kx = classify(x);

@@ -46,11 +46,18 @@ def _addr(a) -> int | None:
     raise TypeError(f"unsupported array type {type(a)!r}")
 
 
+_DTYPES = {"f8": ("float64",), "i4": ("int32",), "u1": ("uint8", "bool")}
+_dtype_names: dict = {}  # dtype -> its name without "torch."
+
+
 def _check_dtype(a, kind: str) -> None:
     if a is None:
         return
-    want = {"f8": ("float64",), "i4": ("int32",), "u1": ("uint8", "bool")}[kind]
-    name = str(a.dtype).replace("torch.", "")
+    want = _DTYPES[kind]
+    name = _dtype_names.get(a.dtype)
+    if name is None:
+        name = str(a.dtype).replace("torch.", "")
+        _dtype_names[a.dtype] = name
     if name not in want:
         raise TypeError(f"expected dtype {want[0]}, got {name}")
 
@@ -107,6 +114,17 @@ class PlacedVolume:
               aux=None, daughter: int = 0, precision: int = L.PREC_FP64, stream=None) -> None:
         g = self.geometry
         g._require_closed()
+        s = stream.cuda_stream if hasattr(stream, "cuda_stream") else stream
+        # plain tensors go through one native call; it leaves everything else, errors
+        # included, to the general path below
+        if hasattr(points.x, "data_ptr"):
+            st = L.pycall().batch(
+                *g._batch_call(), self.id, op, points.x, points.y, points.z,
+                dirs.x if dirs is not None else None, dirs.y if dirs is not None else None,
+                dirs.z if dirs is not None else None, step_max, out, aux, daughter, precision, s)
+            if st is not None:
+                check(st)
+                return
         n = points.size()
         if _len(out) < n:
             raise ValueError("output shorter than the batch")
@@ -116,7 +134,6 @@ class PlacedVolume:
             _check_dtype(step_max, "f8")
         _check_dtype(aux, "i4")
         d = dirs
-        s = stream.cuda_stream if hasattr(stream, "cuda_stream") else stream
         check(g.L.vgb_batch(
             g.handle, self.id, op, n, _addr(points.x), _addr(points.y), _addr(points.z),
             _addr(d.x) if d else None, _addr(d.y) if d else None, _addr(d.z) if d else None,
@@ -215,6 +232,15 @@ class Geometry:
         out = ctypes.c_int32()
         check(fn(self.handle, *args, ctypes.byref(out)))
         return out.value
+
+    def _batch_call(self):
+        """Addresses of vgb_batch, vgb_batch_device and the geometry, for the native call."""
+        c = self.__dict__.get("_batch_args")
+        if c is None:
+            c = (*(ctypes.cast(f, ctypes.c_void_p).value
+                   for f in (self.L.vgb_batch, self.L.vgb_batch_device)), self.handle.value)
+            self._batch_args = c
+        return c
 
     def _require_closed(self) -> None:
         if not self.closed:
