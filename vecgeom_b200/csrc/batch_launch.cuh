@@ -14,6 +14,23 @@
 
 namespace vgb {
 
+// Launches a batch kernel so that its set-up overlaps the end of the batch kernel before
+// it in the stream (batch_kernel_begin).
+template <class... K, class... A>
+void launch_overlapped(void (*k)(K...), dim3 grid, size_t smem, cudaStream_t s, const A &...a) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = dim3(kBatchBlock);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, a...);
+}
+
 inline int grid_for(int64_t n) {
   // enough CTAs to fill 148 SMs x 8 resident 256-thread CTAs; grid-stride beyond
   const int64_t want = (n + kBatchBlock - 1) / kBatchBlock;
@@ -51,9 +68,9 @@ vgb_status BatchLaunch<Ops, P>::batch(const P &prm, const DXform &X, int op, Bat
   switch (op) {
 #define VGB_OP_CASE(OPC)                                                      \
   case OPC:                                                                   \
-    k_batch<Ops, P, OPC><<<RegroupedWalk<Ops, OPC>::value ? std::min(grid, kWalkGridCap) \
-                                                          : grid,                    \
-                           kBatchBlock, smem, s>>>(prm, X, io);                      \
+    launch_overlapped(k_batch<Ops, P, OPC>,                                   \
+                      RegroupedWalk<Ops, OPC>::value ? std::min(grid, kWalkGridCap) : grid, smem, \
+                      s, prm, X, io);                                         \
     break;
     VGB_OP_CASE(VGB_OP_CONTAINS)
     VGB_OP_CASE(VGB_OP_INSIDE)
@@ -85,10 +102,10 @@ vgb_status BatchLaunch<Ops, P>::fused(const P &prm, const DXform &X, const Fused
     const int32_t stage =
         (Stageable<P>::value && rec_len > 0 && rec_len <= kStageMaxDoubles) ? rec_len : 0;
     const dim3 grid(std::min(grid_for(io.n), kWalkGridCap), groups);
-    k_fused_split<Ops, P>
-        <<<grid, kBatchBlock, (size_t)stage * sizeof(double), s>>>(prm, X, io, stage);
+    launch_overlapped(k_fused_split<Ops, P>, grid, (size_t)stage * sizeof(double), s, prm, X, io,
+                      stage);
   } else {
-    k_fused<Ops, P><<<grid_for(io.n), kBatchBlock, 0, s>>>(prm, X, io);
+    launch_overlapped(k_fused<Ops, P>, dim3(grid_for(io.n)), 0, s, prm, X, io);
   }
   count_launch();
   cudaError_t e = cudaGetLastError();
