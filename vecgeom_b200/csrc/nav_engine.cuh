@@ -12,7 +12,9 @@
 // counting sort over 32 classes, a few dozen instructions a track against the
 // thousands of a step.  The tracks in wide volumes (hundreds of daughters) are the
 // last class: each is stepped by a whole warp, which searches the daughters' boxes
-// 32 at a time, so no thread holds its block up for a long list.  A finished track's slot takes the next track of the block's
+// 32 at a time, so no thread holds its block up for a long list; the warps take these
+// tracks one by one as they finish their threads' steps (a fixed share each kept the
+// block waiting: traces of 65,536 detector tracks 3,226 us, now 3,102).  A finished track's slot takes the next track of the block's
 // stream (grid-stride), so blocks stay full while tracks are left.
 #pragma once
 #include "navigation.cuh"
@@ -50,6 +52,7 @@ struct NavPool {
   int32_t v[kNavMaxLevels][kEngThreads];
   int32_t count[kEngThreads];  // tracks per (class, warp), then their first places
   int32_t wsum[kEngWarps];
+  int32_t next;  // the next track of the last class that a warp takes
   uint8_t boundary[kEngThreads];
   uint8_t key[kEngThreads];
   uint8_t order[kEngThreads];
@@ -88,6 +91,7 @@ VGB_D int pool_sort(NavPool &S) {
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   __syncthreads();  // the last step's slots are written, its places read
   S.count[t] = 0;
+  if (t == 0) S.next = 0;
   __syncthreads();
   const int key = S.key[t];
   const unsigned m = __match_any_sync(0xffffffffu, key);
@@ -147,7 +151,19 @@ VGB_D void nav_engine(const NavGeom &G, const C &client, int64_t n) {
     const int live = pool_sort(S);
     if (live == 0) return;
     const int warp_first = S.count[kEngWarp * kEngWarps];  // first place of the last class
-    for (int j = warp_first + (int)(threadIdx.x >> 5); j < live; j += kEngWarps) {
+    if ((int)threadIdx.x < warp_first) {
+      const int slot = S.order[threadIdx.x];
+      const int64_t i = S.idx[slot];
+      pool_get(S, slot, t);
+      after(slot, i, t, client.template step<OneLane>(G, i, t));
+    }
+    __syncwarp();
+    // the warps share the last class's tracks out as they get done
+    for (;;) {
+      int j = 0;
+      if (lane == 0) j = warp_first + atomicAdd(&S.next, 1);
+      j = __shfl_sync(0xffffffffu, j, 0);
+      if (j >= live) break;
       const int slot = S.order[j];
       const int64_t i = S.idx[slot];
       pool_get(S, slot, t);
@@ -156,12 +172,6 @@ VGB_D void nav_engine(const NavGeom &G, const C &client, int64_t n) {
       if (lane == 0) after(slot, i, t, more);
       __syncwarp();
     }
-    if ((int)threadIdx.x < warp_first) {
-      const int slot = S.order[threadIdx.x];
-      const int64_t i = S.idx[slot];
-      pool_get(S, slot, t);
-      after(slot, i, t, client.template step<OneLane>(G, i, t));
-    }
   }
 }
 
@@ -169,11 +179,11 @@ VGB_D void nav_engine(const NavGeom &G, const C &client, int64_t n) {
 // finishes its track's step sooner (3 us against 25 in the layered detector), a
 // thread's step costs a fifth of the instructions: few tracks go to warps, many to
 // threads.  The lines lie where the two cross.  Measured (B200, us by warps / by
-// threads): detector steps of 8,192 tracks 55 / 88, of 50,021 264 / 124; its traces
-// of 64 steps of 16,384 tracks 1,807 / 1,967, of 65,536 7,756 / 3,226; ABBox traces of
-// 16,384 2,501 / 3,674, of 32,768 5,349 / 4,369.  In mixed shapes a warp runs its
+// threads): detector steps of 8,192 tracks 55 / 88, of 50,021 264 / 108; its traces
+// of 64 steps of 16,384 tracks 1,807 / 1,950, of 65,536 7,756 / 3,102; ABBox traces of
+// 16,384 2,501 / 3,674, of 32,768 5,349 / 4,135.  In mixed shapes a warp runs its
 // daughters' different code one after the other, a class of threads walks one list:
-// steps of 1,024 tracks 63 / 227, of 8,192 347 / 243, of 50,021 3,087 / 594; traces of
+// steps of 1,024 tracks 63 / 227, of 8,192 347 / 243, of 50,021 3,087 / 493; traces of
 // 16,384 6,315 / 8,258, of 65,536 24,506 / 20,936; ABBox traces of 1,024 1,171 / 6,053,
 // of 16,384 11,199 / 6,964.
 enum class NavCall { kLocate, kStep, kTrace, kAbboxStep, kAbboxTrace };
