@@ -25,6 +25,10 @@ using namespace vgb;
 
 namespace vgb {
 namespace {
+struct BasketIO : FusedIO {};
+}  // namespace
+template <> struct ReadOnlyInputs<BasketIO> : std::true_type {};
+namespace {
 
 struct BasketRec {
   int32_t unplaced;
@@ -51,7 +55,7 @@ template <> struct HasBase<BooleanP> : std::true_type {};
 // switch over every shape would spill)
 template <class Ops, class P, int kBlock, uint32_t kOps, bool kRegroup = false>
 __device__ __forceinline__ void run_tile(const double *rec, const DXform *xg, int64_t first,
-                                         int64_t end, const FusedIO &io, double *srec,
+                                         int64_t end, const BasketIO &io, double *srec,
                                          DXform *sx) {
   static_assert(sizeof(P) <= kRecDoubles * sizeof(double), "shape record too large to stage");
   constexpr int nd = (int)((sizeof(P) + 7) / 8);
@@ -71,7 +75,7 @@ __device__ __forceinline__ void run_tile(const double *rec, const DXform *xg, in
     if ((io.ops & kDtiSti) == kDtiSti) {
       double *sti = static_cast<double *>(io.out[VGB_OP_SAFETY_TO_IN]);
       for (int64_t i = first + threadIdx.x; i < end; i += kBlock) {
-        const V3<double> m = {ldg(io.x + i), ldg(io.y + i), ldg(io.z + i)};
+        const V3<double> m = {ldg<BasketIO>(io.x + i), ldg<BasketIO>(io.y + i), ldg<BasketIO>(io.z + i)};
         sti[i] = Ops::safety_to_in(prm, xf_point(*sx, m));
       }
       const int64_t base = first + 32 * (threadIdx.x >> 5);
@@ -96,7 +100,7 @@ template <int kBlock, uint32_t kOps>
 __global__ void __launch_bounds__(kBlock, 1)
     k_baskets(const BasketGeom G, const BasketRec *__restrict__ baskets,
               const int64_t *__restrict__ prefix, int32_t nb, int64_t ntiles, int32_t tile,
-              const FusedIO io) {
+              const BasketIO io) {
   __shared__ __align__(16) double srec[kRecDoubles];
   __shared__ DXform sx;
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
@@ -132,7 +136,7 @@ template <class Ops, class P, int kBlock, uint32_t kOps>
 __global__ void __launch_bounds__(kBlock)
     k_baskets_kind(const BasketGeom G, const BasketRec *__restrict__ baskets,
                    const int64_t *__restrict__ prefix, int32_t b0, int32_t b1, int64_t t0,
-                   int64_t t1, int32_t tile, const FusedIO io) {
+                   int64_t t1, int32_t tile, const BasketIO io) {
   __shared__ __align__(16) double srec[kRecDoubles];
   __shared__ DXform sx;
   for (int64_t t = t0 + blockIdx.x; t < t1; t += gridDim.x) {
@@ -224,10 +228,10 @@ vgb_status set_tile(vgb_basket_plan *p, int32_t tile, cudaStream_t s) {
   return VGB_OK;
 }
 
-FusedIO make_io(const vgb_basket_plan *p, const double *x, const double *y, const double *z,
+BasketIO make_io(const vgb_basket_plan *p, const double *x, const double *y, const double *z,
                 const double *dx, const double *dy, const double *dz, const double *step,
                 void *const *outs, uint32_t flags) {
-  FusedIO io;
+  BasketIO io;
   std::memset(&io, 0, sizeof(io));
   io.x = x; io.y = y; io.z = z;
   io.dx = dx; io.dy = dy; io.dz = dz;
@@ -240,7 +244,7 @@ FusedIO make_io(const vgb_basket_plan *p, const double *x, const double *y, cons
 }
 
 template <uint32_t kOps, int kBlock, class Ops, class P>
-void launch_kind_t(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, const FusedIO &io,
+void launch_kind_t(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, const BasketIO &io,
                    cudaStream_t s) {
   const BasketGeom G = {p->g->dev.params, p->g->dev.unplaced, p->g->dev.xforms};
   int dev = 0, sms = 148, per_sm = 1;
@@ -262,7 +266,7 @@ void launch_kind_t(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, con
 constexpr int32_t kKindPairBox = 1, kKindPairBoxTube = 2;
 
 template <uint32_t kOps, int kBlock>
-void launch_kind(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, const FusedIO &io,
+void launch_kind(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, const BasketIO &io,
                  cudaStream_t s) {
   if (k.type == VGB_SHAPE_BOOLEAN) {
     if (k.sub == kKindPairBoxTube)
@@ -283,7 +287,7 @@ void launch_kind(const vgb_basket_plan *p, const vgb_basket_plan::Kind &k, const
 }
 
 template <uint32_t kOps>
-void launch_kinds(const vgb_basket_plan *p, const FusedIO &io, cudaStream_t s) {
+void launch_kinds(const vgb_basket_plan *p, const BasketIO &io, cudaStream_t s) {
   const int nk = (int)p->kinds.size();
   if (nk > 1) cudaEventRecord(p->kfork, s);
   for (int i = 0; i < nk; ++i) {
@@ -298,7 +302,7 @@ void launch_kinds(const vgb_basket_plan *p, const FusedIO &io, cudaStream_t s) {
   for (int i = 1; i < nk; ++i) cudaStreamWaitEvent(s, p->kjoin[i - 1], 0);
 }
 
-vgb_status launch(const vgb_basket_plan *p, const FusedIO &io, cudaStream_t s) {
+vgb_status launch(const vgb_basket_plan *p, const BasketIO &io, cudaStream_t s) {
   if (p->ntiles == 0) return VGB_OK;
   if ((p->ops & ~kOpsDtiSti) == 0)
     launch_kinds<kOpsDtiSti>(p, io, s);
@@ -466,7 +470,7 @@ vgb_status vgb_basket_tune(vgb_basket_plan *p, const double *x, const double *y,
   if (s != VGB_OK) return s;
   if (reps < 1) reps = 1;
   cudaStream_t st = (cudaStream_t)stream;
-  const FusedIO io = make_io(p, x, y, z, dx, dy, dz, step_max, outs, flags);
+  const BasketIO io = make_io(p, x, y, z, dx, dy, dz, step_max, outs, flags);
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
@@ -637,7 +641,7 @@ __global__ void __launch_bounds__(1024)
 
 template <uint32_t kOps>
 void noalloc_launch(const vgb_geometry *g, const BasketRec *rec, const int64_t *prefix,
-                    int32_t nb, int64_t ntiles, const FusedIO &io, cudaStream_t s) {
+                    int32_t nb, int64_t ntiles, const BasketIO &io, cudaStream_t s) {
   const BasketGeom G = {g->dev.params, g->dev.unplaced, g->dev.xforms};
   static_assert(kNoallocBlock == 256, "the all-shape kernel is built for 256-thread CTAs");
   const int grid = (int)std::min<int64_t>(ntiles, occupancy_grid<kOps>());
@@ -698,7 +702,7 @@ extern "C" vgb_status vgb_basket_run_noalloc(const vgb_geometry *g, const vgb_ba
   }
   if (e != cudaSuccess) return cuda_error(e, "vgb_basket_run_noalloc: basket copy");
   k_noalloc_tables<<<1, 1024, 0, s>>>(raw, nb, g->dev.placed, kNoallocTile, rec, prefix);
-  FusedIO io;
+  BasketIO io;
   std::memset(&io, 0, sizeof(io));
   io.x = x; io.y = y; io.z = z;
   io.dx = dx; io.dy = dy; io.dz = dz;
