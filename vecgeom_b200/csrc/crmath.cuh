@@ -27,7 +27,7 @@
 // strategy): sin and cos of the nearest multiple of pi/64 from a table of 32
 // double-doubles, the remainder's series in double behind its leading terms, good to
 // about 2^-66.  When the value less and plus its error bound rounds to one double,
-// that is the correctly rounded result; otherwise (about one call in 2^10) the series
+// that is the correctly rounded result; otherwise (about one call in 2^13) the series
 // above decides.  The two evaluate the same function, so no result depends on which
 // one answered.  The series costs ~800 operations a call, the short form ~100: torus
 // DistanceToIn on 2^22 mixed rays 657 -> 322 us, DistanceToOut on 2^21 295 -> 122 us.
@@ -207,20 +207,25 @@ VGB_HD void sincos_reduced(DD r, DD &s, DD &c) {
     {0x1.fa7557f08a517p-1, -0x1.7a0a8ca13571fp-55, 0x1.2c8106e8e613ap-3, 0x1.13000a89a11e0p-58}, \
     {0x1.fd88da3d12526p-1, -0x1.87df6378811c7p-55, 0x1.917a6bc29b42cp-4, -0x1.e2718d26ed688p-60}, \
     {0x1.ff621e3796d7ep-1, -0x1.c57bc2e24aa15p-57, 0x1.91f65f10dd814p-5, -0x1.912bd0d569a90p-61}
+// The device reads a row as two 16-byte words, so the row's type asks for that
+// alignment: a table of plain doubles is placed on 8 bytes.
+struct alignas(16) SinCosEntry {
+  double v[4];
+};
 #ifdef __CUDACC__
-static __device__ const double kCrmSinCosDev[32][4] = {VGB_CRM_SINCOS_ROWS};
+static __device__ const SinCosEntry kCrmSinCosDev[32] = {VGB_CRM_SINCOS_ROWS};
 #endif
-static const double kCrmSinCosHost[32][4] = {VGB_CRM_SINCOS_ROWS};
+static const SinCosEntry kCrmSinCosHost[32] = {VGB_CRM_SINCOS_ROWS};
 struct SinCosRow {
   DD s, c;
 };
 VGB_HD SinCosRow sincos_row(int j) {
 #ifdef __CUDA_ARCH__
-  const double2 *r = reinterpret_cast<const double2 *>(kCrmSinCosDev[j]);
+  const double2 *r = reinterpret_cast<const double2 *>(kCrmSinCosDev[j].v);
   const double2 a = __ldg(r), b = __ldg(r + 1);
   return {{a.x, a.y}, {b.x, b.y}};
 #else
-  const double *r = kCrmSinCosHost[j];
+  const double *r = kCrmSinCosHost[j].v;
   return {{r[0], r[1]}, {r[2], r[3]}};
 #endif
 }
