@@ -362,43 +362,68 @@ struct BoxItem {
 // size, at most 64 along an axis.  A point's cell and a box's cells come from the
 // same float expression, which is monotone, so a box's range holds the cell of
 // every point of the box.
+// Small daughters far apart would make most cells empty, and large ones fill every cell,
+// so the longest axis is halved until there are no more than kCellsPerDaughter cells and
+// as many list entries a daughter: the tables grow with the daughters, by at most the
+// size of two of their NavSlots each (the layered detector's layers have 2 to 25 of
+// both).  One cell would be the whole list: no grid then (0).
+constexpr int64_t kCellsPerDaughter = 32;
 int32_t build_grid(vgb_geometry *g, const std::vector<BoxItem> &it) {
   CellGrid c = {};
-  float hi[3];
+  double extent[3];
   for (int k = 0; k < 3; ++k) {
+    float hi = -3e38f;
     c.org[k] = 3e38f;
-    hi[k] = -3e38f;
     double size = 0.;
     for (const BoxItem &b : it) {
       c.org[k] = std::min(c.org[k], b.lo[k]);
-      hi[k] = std::max(hi[k], b.hi[k]);
+      hi = std::max(hi, b.hi[k]);
       size += (double)b.hi[k] - b.lo[k];
     }
-    const double extent = (double)hi[k] - c.org[k];
-    const double cells = std::ceil(extent / (0.5 * size / it.size()));
+    extent[k] = (double)hi - c.org[k];
+    const double cells = std::ceil(extent[k] / (0.5 * size / it.size()));
     c.n[k] = (int32_t)std::min(64., std::max(1., cells));
-    c.inv[k] = (float)(c.n[k] / (extent * (1. + 1e-5)));  // the last box ends inside the grid
   }
-  c.first = (int32_t)g->cell_start.size();
-  // counted first, then filled in daughter order
-  const size_t ncell = (size_t)c.n[0] * c.n[1] * c.n[2];
-  auto each_cell = [&](const BoxItem &b, auto f) {
-    int a[3], z[3];
+  // the cells of a box, first and last along each axis
+  auto range = [&](const BoxItem &b, int a[3], int z[3]) {
     for (int k = 0; k < 3; ++k) {
       a[k] = cell_of(c, k, b.lo[k]);
       z[k] = std::min(cell_of(c, k, b.hi[k]), c.n[k] - 1);
     }
+  };
+  const int64_t most = std::min<int64_t>(kCellsPerDaughter * (int64_t)it.size(), INT32_MAX);
+  for (;;) {
+    for (int k = 0; k < 3; ++k)
+      c.inv[k] = (float)(c.n[k] / (extent[k] * (1. + 1e-5)));  // the last box ends inside the grid
+    int64_t entries = 0;
+    for (const BoxItem &b : it) {
+      int a[3], z[3];
+      range(b, a, z);
+      entries += (int64_t)(z[0] - a[0] + 1) * (z[1] - a[1] + 1) * (z[2] - a[2] + 1);
+    }
+    if ((int64_t)c.n[0] * c.n[1] * c.n[2] <= most && entries <= most) break;
+    int32_t *n = std::max_element(c.n, c.n + 3);
+    *n = (*n + 1) / 2;
+  }
+  const size_t ncell = (size_t)c.n[0] * c.n[1] * c.n[2];
+  if (ncell == 1) return 0;
+  c.first = (int64_t)g->cell_start.size();
+  c.items = (int64_t)g->cell_items.size();
+  // counted first, then filled in daughter order
+  auto each_cell = [&](const BoxItem &b, auto f) {
+    int a[3], z[3];
+    range(b, a, z);
     for (int iz = a[2]; iz <= z[2]; ++iz)
       for (int iy = a[1]; iy <= z[1]; ++iy)
         for (int ix = a[0]; ix <= z[0]; ++ix) f(((size_t)iz * c.n[1] + iy) * c.n[0] + ix);
   };
   std::vector<int32_t> at(ncell + 1, 0);
   for (const BoxItem &b : it) each_cell(b, [&](size_t k) { ++at[k + 1]; });
-  at[0] = (int32_t)g->cell_items.size();
   for (size_t k = 0; k < ncell; ++k) at[k + 1] += at[k];
   g->cell_start.insert(g->cell_start.end(), at.begin(), at.end());
-  g->cell_items.resize(at[ncell]);
-  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { g->cell_items[at[k]++] = b.d; });
+  g->cell_items.resize(c.items + at[ncell]);
+  int32_t *items = g->cell_items.data() + c.items;
+  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { items[at[k]++] = b.d; });
   g->grids.push_back(c);
   return (int32_t)g->grids.size();
 }
