@@ -5,13 +5,13 @@
 // converting sixteen ctypes arguments and asking the driver what kind of memory two of
 // them are took the host 9.6 (four Python calls a tensor, 1 us a driver query; now 3.8,
 // of which the launch is more than half).  batch() does the first two here, from the tensors'
-// own fields, and calls vgb_batch_device where the tensors say that they are on a GPU.
+// own fields, and calls vgb_batch_device where the tensors say that they are all on one GPU.
 //
 // It handles the plain case only: every array a torch.Tensor itself, contiguous, with
-// the lengths and types the call needs.  For anything else (numpy arrays, subclasses,
-// tensors without storage, a wrong length, an empty batch) it returns None without
-// calling, and the caller's general path does the call or raises its errors.  Nothing
-// is kept between calls.
+// the lengths and types the call needs, and all of them on one device.  For anything
+// else (numpy arrays, subclasses, tensors without storage, a wrong length, a mix of
+// devices, an empty batch) it returns None without calling, and the caller's general
+// path does the call or raises its errors.  Nothing is kept between calls.
 #include <Python.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -56,8 +56,9 @@ PyObject *batch(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     if (a[11] != Py_None && ok) ok = (t[6] = plain(a[11], n, true, &f8));
     if (ok) ok = (t[7] = plain(a[12], n, true, nullptr));
     if (a[13] != Py_None && ok) ok = (t[8] = plain(a[13], n, true, &i4));
+    for (int k = 1; k < 9 && ok; ++k) ok = !t[k] || t[k]->device() == t[0]->device();
     if (!ok) Py_RETURN_NONE;
-    const bool device = t[0]->is_cuda() && t[7]->is_cuda();
+    const bool device = t[0]->is_cuda();
     const auto fn = reinterpret_cast<BatchFn>(PyLong_AsVoidPtr(a[device ? 1 : 0]));
     const auto g = static_cast<const vgb_geometry *>(PyLong_AsVoidPtr(a[2]));
     const long placed = PyLong_AsLong(a[3]), op = PyLong_AsLong(a[4]);

@@ -66,6 +66,25 @@ def _len(a) -> int:
     return int(a.shape[0])
 
 
+def _check_reachable(x, out, *arrays) -> None:
+    """Where x is on a GPU the kernels read and write every array in place: each has to be
+    on the same GPU or in pinned host memory.  (An output in any host memory is left to
+    the library, which refuses it beside a device input.)"""
+    if not getattr(x, "is_cuda", False):
+        return
+    for a in (out, *arrays):
+        if a is None or getattr(a, "device", None) == x.device:
+            continue
+        if isinstance(a, np.ndarray) and a is not out:
+            import torch
+            a = torch.from_numpy(a)
+        # (an array type of its own says nothing of where it is)
+        if not getattr(a, "is_cuda", False) and (a is out or not hasattr(a, "is_pinned")
+                                                 or a.is_pinned()):
+            continue
+        raise ValueError("arrays of one call must be on one device")
+
+
 class SOA3D:
     """Structure-of-arrays batch of 3-vectors (base/SOA3D.h:32-39)."""
 
@@ -134,6 +153,9 @@ class PlacedVolume:
             _check_dtype(step_max, "f8")
         _check_dtype(aux, "i4")
         d = dirs
+        if n > 0:
+            _check_reachable(points.x, out, points.y, points.z, *((d.x, d.y, d.z) if d else ()),
+                             step_max, aux)
         check(g.L.vgb_batch(
             g.handle, self.id, op, n, _addr(points.x), _addr(points.y), _addr(points.z),
             _addr(d.x) if d else None, _addr(d.y) if d else None, _addr(d.z) if d else None,
