@@ -279,7 +279,9 @@ vgb_status vgb_SafetyToOut(const vgb_geometry *g, int32_t placed, int64_t n, con
  * call covers what a caller would otherwise run as two (all points, then the
  * inside subset).  Buffers are all device or all host memory; host buffers
  * cross to the device once per chunk for all the requested ops (staged as in
- * vgb_batch), and the call returns with the outputs written. */
+ * vgb_batch), and the call returns with the outputs written.
+ * A double output may be one of the call's input arrays: a point's inputs are
+ * all read before its outputs are written. */
 enum { VGB_FUSED_DTO_INSIDE_ONLY = 1, VGB_FUSED_LOCAL_INSIDE_ONLY = 2 };
 vgb_status vgb_batch_fused(const vgb_geometry *g, int32_t placed, uint32_t ops, int64_t n,
                            const double *x, const double *y, const double *z, const double *dx,

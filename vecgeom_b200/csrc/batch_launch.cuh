@@ -93,20 +93,43 @@ vgb_status BatchLaunch<Ops, P>::batch(const P &prm, const DXform &X, int op, Bat
   return VGB_OK;
 }
 
+// Whether an output of a fused call shares memory with one of the inputs it reads.
+inline bool fused_in_place(const FusedIO &io) {
+  const double *in[] = {io.x, io.y, io.z, io.dx, io.dy, io.dz, io.step};
+  const bool dirs = io.ops & ((1u << VGB_OP_DISTANCE_TO_IN) | (1u << VGB_OP_DISTANCE_TO_OUT));
+  for (int op = 0; op < 6; ++op) {
+    if (!((io.ops >> op) & 1u)) continue;
+    const uintptr_t size = op == VGB_OP_CONTAINS ? 1 : op == VGB_OP_INSIDE ? 4 : 8;
+    const uintptr_t o = reinterpret_cast<uintptr_t>(io.out[op]), oe = o + size * io.n;
+    for (int k = 0; k < (dirs ? 7 : 3); ++k) {
+      const uintptr_t i = reinterpret_cast<uintptr_t>(in[k]);
+      if (o < i + 8 * io.n && i < oe) return true;
+    }
+  }
+  return false;
+}
+
 template <class Ops, class P>
 vgb_status BatchLaunch<Ops, P>::fused(const P &prm, const DXform &X, const FusedIO &io,
                                       cudaStream_t s, int32_t rec_len) {
+  bool rows = false;
   if constexpr (SplitFused<P>::value) {
-    const int groups = (io.ops & kPointOps ? 1 : 0) + (io.ops & (1u << VGB_OP_DISTANCE_TO_IN) ? 1 : 0) +
-                       (io.ops & (1u << VGB_OP_DISTANCE_TO_OUT) ? 1 : 0);
-    const int32_t stage =
-        (Stageable<P>::value && rec_len > 0 && rec_len <= kStageMaxDoubles) ? rec_len : 0;
-    const dim3 grid(std::min(grid_for(io.n), kWalkGridCap), groups);
-    launch_overlapped(k_fused_split<Ops, P>, grid, (size_t)stage * sizeof(double), s, prm, X, io,
-                      stage);
-  } else {
-    launch_overlapped(k_fused<Ops, P>, dim3(grid_for(io.n)), 0, s, prm, X, io);
+    // the rows of a call read the inputs independently of each other's stores, so a call
+    // that writes an output over one of its inputs takes the kernel whose threads read a
+    // point's inputs before they store
+    rows = !fused_in_place(io);
+    if (rows) {
+      const int groups = (io.ops & kPointOps ? 1 : 0) +
+                         (io.ops & (1u << VGB_OP_DISTANCE_TO_IN) ? 1 : 0) +
+                         (io.ops & (1u << VGB_OP_DISTANCE_TO_OUT) ? 1 : 0);
+      const int32_t stage =
+          (Stageable<P>::value && rec_len > 0 && rec_len <= kStageMaxDoubles) ? rec_len : 0;
+      const dim3 grid(std::min(grid_for(io.n), kWalkGridCap), groups);
+      launch_overlapped(k_fused_split<Ops, P>, grid, (size_t)stage * sizeof(double), s, prm, X, io,
+                        stage);
+    }
   }
+  if (!rows) launch_overlapped(k_fused<Ops, P>, dim3(grid_for(io.n)), 0, s, prm, X, io);
   count_launch();
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_error(e, "vgb_batch_fused: kernel launch");
