@@ -7,10 +7,13 @@ is no CPU fallback for any operation.
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
+import sys
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "lib", "libvgb.so")
+PYCALL_PATH = os.path.join(_HERE, "lib", "_pycall.so")
 
 # vgb_status (include/vgb.h)
 OK, EINVAL, ENOMEM, ECUDA, ELOOPCAP, ETIMEDOUT, ENOTSUP, ENOSPC = range(8)
@@ -158,24 +161,40 @@ def lib():
     return L
 
 
-_pycall = None
+_pycall = None  # the module, or False where it cannot be used
 
 
 def pycall():
-    """The native call module (csrc/pycall.cpp), which links to the torch libraries of
-    the running process (called with tensors in hand); raises if it was not built."""
+    """The native call module (csrc/pycall.cpp), or None where it cannot be used: not
+    built, built for another torch or Python, or torch is not loaded in this process (it
+    links to the process's torch libraries).  The calls it serves have a general path."""
     global _pycall
     if _pycall is None:
-        import importlib.util
-        path = os.path.join(_HERE, "lib", "_pycall.so")
-        if not os.path.exists(path):
-            raise ImportError(f"_pycall.so not found at {path}: build it with "
-                              "`make -C vecgeom_b200/csrc` (or __graft_entry__.build())")
-        spec = importlib.util.spec_from_file_location("_pycall", path)
-        m = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(m)
-        _pycall = m
-    return _pycall
+        torch = sys.modules.get("torch")
+        if torch is None:
+            return None
+        try:
+            spec = importlib.util.spec_from_file_location("_pycall", PYCALL_PATH)
+            m = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(m)
+            _pycall = m if m.torch_version == str(torch.__version__) else False
+        except (ImportError, OSError, AttributeError):
+            _pycall = False
+    return _pycall or None
+
+
+def batch_entries(L):
+    """Addresses of a library's vgb_batch and vgb_batch_device, looked up once per
+    library; None for a handle that lacks either."""
+    e = getattr(L, "_batch_entries", False)
+    if e is False:
+        try:
+            e = tuple(ctypes.cast(f, ctypes.c_void_p).value
+                      for f in (L.vgb_batch, L.vgb_batch_device))
+        except (AttributeError, ctypes.ArgumentError):
+            e = None
+        L._batch_entries = e
+    return e
 
 
 def check(status: int) -> None:

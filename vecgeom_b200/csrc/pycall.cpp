@@ -12,12 +12,19 @@
 // else (numpy arrays, subclasses, tensors without storage, a wrong length, a mix of
 // devices, an empty batch) it returns None without calling, and the caller's general
 // path does the call or raises its errors.  Nothing is kept between calls.
+//
+// The module is only good for the torch and the Python it was built with: it names the
+// one (torch_version) for its loader to compare and refuses to load in another of the other.
 #include <Python.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstdint>
+#include <string>
 
 #include "../../include/vgb.h"
+
+#define VGB_TEXT(x) #x
+#define VGB_TEXT_OF(x) VGB_TEXT(x)
 
 namespace {
 
@@ -92,4 +99,16 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_pycall", nullptr, -1, methods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__pycall() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__pycall() {
+  const std::string built = std::to_string(PY_MAJOR_VERSION) + "." + std::to_string(PY_MINOR_VERSION);
+  if (std::string(Py_GetVersion()).rfind(built + ".", 0) != 0) {
+    PyErr_SetString(PyExc_ImportError, ("built for Python " + built).c_str());
+    return nullptr;
+  }
+  PyObject *m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "torch_version", VGB_TEXT_OF(VGB_TORCH_VERSION)) < 0) {
+    Py_DECREF(m);
+    return nullptr;
+  }
+  return m;
+}

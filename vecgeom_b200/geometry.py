@@ -136,9 +136,11 @@ class PlacedVolume:
         s = stream.cuda_stream if hasattr(stream, "cuda_stream") else stream
         # plain tensors go through one native call; it leaves everything else, errors
         # included, to the general path below
-        if hasattr(points.x, "data_ptr"):
-            st = L.pycall().batch(
-                *g._batch_call(), self.id, op, points.x, points.y, points.z,
+        native = L.pycall() if hasattr(points.x, "data_ptr") else None
+        entries = L.batch_entries(g.L) if native is not None else None
+        if entries is not None:
+            st = native.batch(
+                *entries, g.handle.value, self.id, op, points.x, points.y, points.z,
                 dirs.x if dirs is not None else None, dirs.y if dirs is not None else None,
                 dirs.z if dirs is not None else None, step_max, out, aux, daughter, precision, s)
             if st is not None:
@@ -254,15 +256,6 @@ class Geometry:
         out = ctypes.c_int32()
         check(fn(self.handle, *args, ctypes.byref(out)))
         return out.value
-
-    def _batch_call(self):
-        """Addresses of vgb_batch, vgb_batch_device and the geometry, for the native call."""
-        c = self.__dict__.get("_batch_args")
-        if c is None:
-            c = (*(ctypes.cast(f, ctypes.c_void_p).value
-                   for f in (self.L.vgb_batch, self.L.vgb_batch_device)), self.handle.value)
-            self._batch_args = c
-        return c
 
     def _require_closed(self) -> None:
         if not self.closed:
