@@ -391,11 +391,12 @@ int32_t build_grid(vgb_geometry *g, const std::vector<BoxItem> &it) {
       z[k] = std::min(cell_of(c, k, b.hi[k]), c.n[k] - 1);
     }
   };
-  const int64_t most = std::min<int64_t>(kCellsPerDaughter * (int64_t)it.size(), INT32_MAX);
+  const int64_t most = kCellsPerDaughter * (int64_t)it.size();
+  int64_t entries;
   for (;;) {
     for (int k = 0; k < 3; ++k)
       c.inv[k] = (float)(c.n[k] / (extent[k] * (1. + 1e-5)));  // the last box ends inside the grid
-    int64_t entries = 0;
+    entries = 0;
     for (const BoxItem &b : it) {
       int a[3], z[3];
       range(b, a, z);
@@ -406,9 +407,11 @@ int32_t build_grid(vgb_geometry *g, const std::vector<BoxItem> &it) {
     *n = (*n + 1) / 2;
   }
   const size_t ncell = (size_t)c.n[0] * c.n[1] * c.n[2];
-  if (ncell == 1) return 0;
-  c.first = (int64_t)g->cell_start.size();
-  c.items = (int64_t)g->cell_items.size();
+  // offsets are 32-bit (64-bit ones cost a trace 0.6 %): no grid past their range
+  if (ncell == 1 || g->cell_start.size() + ncell >= INT32_MAX ||
+      g->cell_items.size() + entries >= INT32_MAX)
+    return 0;
+  c.first = (int32_t)g->cell_start.size();
   // counted first, then filled in daughter order
   auto each_cell = [&](const BoxItem &b, auto f) {
     int a[3], z[3];
@@ -419,11 +422,11 @@ int32_t build_grid(vgb_geometry *g, const std::vector<BoxItem> &it) {
   };
   std::vector<int32_t> at(ncell + 1, 0);
   for (const BoxItem &b : it) each_cell(b, [&](size_t k) { ++at[k + 1]; });
+  at[0] = (int32_t)g->cell_items.size();
   for (size_t k = 0; k < ncell; ++k) at[k + 1] += at[k];
   g->cell_start.insert(g->cell_start.end(), at.begin(), at.end());
-  g->cell_items.resize(c.items + at[ncell]);
-  int32_t *items = g->cell_items.data() + c.items;
-  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { items[at[k]++] = b.d; });
+  g->cell_items.resize(at[ncell]);
+  for (const BoxItem &b : it) each_cell(b, [&](size_t k) { g->cell_items[at[k]++] = b.d; });
   g->grids.push_back(c);
   return (int32_t)g->grids.size();
 }

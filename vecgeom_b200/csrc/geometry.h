@@ -56,15 +56,14 @@ enum : int32_t {
 };
 
 // A grid of equal cells over a volume's daughters: cell c lists, in ascending
-// order, the positions of the daughters whose box meets it: items[this->items +
-// start[first + c] .. + start[first + c + 1]).  Cells are numbered x fastest.
+// order, the positions of the daughters whose box meets it (items[start[first + c]
+// .. start[first + c + 1])).  Cells are numbered x fastest.
 struct CellGrid {
   float org[3];    // lower corner
   float inv[3];    // cells per mm
   int32_t n[3];    // cells per axis
-  int32_t pad;
-  int64_t first;   // of the grid's cells in the start table
-  int64_t items;   // of the grid's lists in the list table
+  int32_t first;   // of the grid's cells in the start table
+  int32_t pad[2];
 };
 VGB_HD int cell_of(const CellGrid &c, int k, float v) {
   return (int)floorf((v - c.org[k]) * c.inv[k]);

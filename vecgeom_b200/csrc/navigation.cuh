@@ -588,7 +588,7 @@ VGB_HD const int32_t *cell_list(const NavGeom &G, const NavVol &lr, const V3<dou
   }
   const int32_t b = st[at];
   count = st[at + 1] - b;
-  return G.cell_items + c.items + b;
+  return G.cell_items + b;
 }
 
 // ---------------------------------------------------------------------------
