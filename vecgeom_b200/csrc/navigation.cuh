@@ -676,9 +676,9 @@ template <class L, uint32_t kMask, bool kScreen = false> struct Navigator {
 
   // The daughters of a wide volume, by a warp: the lanes test 32 boxes at a time and
   // queue the daughters that may lower the safety or the distance; the queue is
-  // evaluated 32 at a time (both answers from one frame change), and what it finds
-  // tightens the tests that follow.  sf and best enter as the mother's values (sf
-  // is not NaN when want_s), hit is the position behind best.  Before, every daughter
+  // evaluated 32 at a time (the answers asked for, both from one frame change), and what
+  // it finds tightens the tests that follow.  sf and best enter as the mother's values (a
+  // NaN sf stays), hit is the position behind best.  Before, every daughter
   // was evaluated: traces of 16 to 1,024 detector tracks by warps 297-380 us with the
   // cells alone, 243-281 with this search.
   static VGB_HD void search_wide(const NavGeom &G, const NavVol &lr, const V3<R> &lp,
@@ -710,8 +710,11 @@ template <class L, uint32_t kMask, bool kScreen = false> struct Navigator {
         int ti = 0x7fffffff, di = 0x7fffffff;
         if (L::lane() < take) {
           const int e = queue[L::lane()];
-          R ts;
-          const R v = S::safety_and_distance_to_in(G, lr.dfirst + e, lp, ld, smax, ts);
+          R ts = Lim<R>::inf(), v;
+          if (want_s)
+            v = S::safety_and_distance_to_in(G, lr.dfirst + e, lp, ld, smax, ts, want_d);
+          else
+            v = S::distance_to_in(G, lr.dfirst + e, lp, ld, smax);
           if (want_s && ts == ts) {
             t = ts;
             ti = e;
