@@ -545,7 +545,9 @@ VGB_HD bool wide_meets(const float4 &lo4, const float4 &hi4, const WidePoint &t,
     tf = l.flat[k] ? tf : fminf(tf, fmaxf(t1, t2));
   }
   out |= tn - tf > 1e-5f * (fabsf(tn) + fabsf(tf));
-  const float bf = best < 3.0e38 ? (float)best : 3.0e38f;
+  // a negative best bounds nothing: a daughter that the point is in answers -1, however
+  // far behind the point its box begins
+  const float bf = best < 3.0e38 ? fmaxf((float)best, 0.f) : 3.0e38f;
   out |= tn > bf * 1.0001f + 1e-3f;
   return !out;
 }
