@@ -33,3 +33,15 @@ def test_an_inside_answer_beats_a_hit_behind_the_point(ws, what):
     d = np.array([[-2e-10], [1.], [0.]])
     want, got = (from_world(ws, g, p, d, boxes, what)[0] for boxes in (0, 1))
     assert got == want
+
+
+@pytest.mark.parametrize("what", [0, 2])
+@pytest.mark.parametrize("unit", [1., 1e6, 1e16, 1e20])
+def test_safeties_at_any_scale(ws, what, unit):
+    g = world(ws, 1000. * unit, [((50. * unit,) * 3, (500. * unit, 10. * unit, 0.))],
+              ((10. * unit,) * 3, 700. * unit))
+    rng = np.random.default_rng(2)
+    p = np.ascontiguousarray(rng.uniform(-300., 300., (3, 200)) * unit)
+    d = np.ascontiguousarray(W.isotropic(rng, 200))
+    want, got = (from_world(ws, g, p, d, boxes, what)[0] for boxes in (0, 1))
+    assert got == want

@@ -561,9 +561,8 @@ VGB_HD bool wide_near(const float4 &lo, const float4 &hi, const WidePoint &t, do
     const float g = fmaxf(fmaxf(a, b), 0.f);
     d2 += g * g;
   }
-  const float bf = best < 1.0e18 ? (float)best : 1.0e18f;
-  const float lim = fmaxf(bf, 0.f) * 1.7323f + 1e-3f;  // sqrt(3) best and a margin
-  return !(d2 > lim * lim);
+  const float lim = fmaxf((float)best, 0.f) * 1.7323f + 1e-3f;  // sqrt(3) best and a margin
+  return !(d2 > lim * lim) || !(best < 1.0e18);  // (d2 and lim * lim stay in a float's range)
 }
 
 // The daughters a point may be in: the list of its cell where the volume has a
