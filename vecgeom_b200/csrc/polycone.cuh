@@ -72,9 +72,10 @@ template <class R> struct PolyconeOps {
     int index, increment;
     R distance;
     // DistanceToIn: what the reachability test needs of the ray, computed once: whether
-    // it applies, 1 / v.z (0: parallel to the planes) and the parameter of the ray's
-    // closest approach to the axis (0 for a ray along it)
-    bool test;
+    // it applies, 1 / v.z (0: parallel to the planes), the parameter of the ray's closest
+    // approach to the axis (0 for a ray along it), and whether the point is so far away
+    // that the planes are reached by divisions
+    bool test, far;
     R invz, tclose;
     // DistanceToOut: the distance so far, the steps taken, the point in the
     // current section's frame
@@ -94,9 +95,11 @@ template <class R> struct PolyconeOps {
     // for any other v (the reference's 0x16A rotation code hands one over) its
     // answers are not points of the surface along the ray, so every section is
     // evaluated; so it is for a point that is not finite
-    const R a = v.x * v.x + v.y * v.y;
-    w.test = fabs(a + v.z * v.z - (R)1) < (R)1e-10 &&
-             fabs(q.x) + fabs(q.y) + fabs(q.z) < Lim<R>::inf();
+    const R a = v.x * v.x + v.y * v.y, size = fabs(q.x) + fabs(q.y) + fabs(q.z);
+    w.test = fabs(a + v.z * v.z - (R)1) < (R)1e-10 && size < Lim<R>::inf();
+    // up to here the rounding of 1 / v.z moves the closest approach by far less than the
+    // margins; beyond, what the test decides is rounding, so it stays that of the divisions
+    w.far = !(size < (R)1e9);
     // a |v.z| below 1e-290 never reaches another slab: parallel to the planes
     w.invz = fabs(v.z) > (R)1e-290 ? (R)1 / v.z : (R)0;
     w.tclose = a > 0 ? -(q.x * v.x + q.y * v.y) / a : (R)0;
@@ -120,7 +123,8 @@ template <class R> struct PolyconeOps {
     // the ray's part in the slab
     R t0 = 0, t1 = Lim<R>::inf();
     if (w.invz != 0) {
-      const R ta = (zlo - q.z) * w.invz, tb = (zhi - q.z) * w.invz;
+      const R ta = w.far ? (zlo - q.z) / v.z : (zlo - q.z) * w.invz;
+      const R tb = w.far ? (zhi - q.z) / v.z : (zhi - q.z) * w.invz;
       t0 = vmax(vmin(ta, tb), (R)0);
       t1 = vmax(ta, tb);
       if (t0 > t1) return true;  // the slab lies behind the point
@@ -143,6 +147,7 @@ template <class R> struct PolyconeOps {
                               Walk &w) {
     bool over = false;
     while (!over && out_of_reach(sec(p, w.index), q, v, w)) {
+      w.distance = Lim<R>::inf();
       w.index += w.increment;
       over = !w.increment || !(w.index >= 0 && w.index < p.nsec);
     }
