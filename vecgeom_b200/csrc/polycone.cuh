@@ -52,7 +52,7 @@ template <class R> struct PolyconeOps {
 
   // ContainsKernel (:52-72)
   static VGB_HD bool contains(const PolyconeP &p, const V3<R> &q) {
-    if (q.z < zs(p, 0) || q.z > zs(p, p.nsec)) return false;
+    if (!(q.z >= zs(p, 0) && q.z <= zs(p, p.nsec))) return false;  // nor is a NaN in a section
     const PolySec &s = sec(p, section_index(p, q.z));
     return C::contains(s.cone, shifted(q, s));
   }
