@@ -12,8 +12,8 @@
 //      locates them (LocatePoint from the world) and clears their counters;
 //   2. step: one launch over the chunks of all admitted requests advances every
 //      live track by up to steps_per_launch steps, each GetSafety and
-//      FindNextBoundaryAndStep (one warp per track, the navigator of
-//      navigation.cuh), and counts the tracks still live per chunk;
+//      FindNextBoundaryAndStep (a warp per track, or with many live ones a
+//      thread, nav_engine.cuh), and counts the tracks still live per chunk;
 //   3. retire: the requests whose chunks have no live track are finished; one
 //      launch gathers their results into a staging buffer, one copy brings them
 //      to pinned host memory, and their chunks are free for the next admission.
@@ -257,6 +257,7 @@ int srv_grid(int64_t ntracks) {
 struct Request {
   int64_t id = -1;
   int64_t n = 0;
+  int64_t live = 0;        // tracks not yet finished after the last step
   int32_t bypassed = 0;    // admissions of later requests while this one waited
   std::vector<double> in;  // x, y, z, dx, dy, dz (6 n)
   std::vector<int32_t> chunks;
@@ -326,8 +327,18 @@ template <uint32_t kMask> void launch_admit(vgb_server *s, int64_t nt) {
   k_srv_admit<kMask><<<srv_grid(nt), kSrvBlock, 0, s->stream>>>(
       server_geom(s->g), s->d_chunks, nt, s->d_in, s->d_valid, s->S, s->g->dev.nav_flags);
 }
-template <uint32_t kMask> void launch_step(vgb_server *s, int64_t nt) {
-  if (nav_by_threads<kMask>(NavCall::kTrace, nt)) {
+// Whether a step over nt slots with `live` unfinished tracks runs by threads.  The slots
+// decide as a trace's tracks do, but with few live tracks among them the thread form's
+// latency is all there is to see: B200, us a step by warps / by threads, 4 steps a launch,
+// detector with 20,480 slots: 477 live 59 / 84, 2,843 live 95 / 106, 5,681 live 125 / 119;
+// 65,536 slots: 1,893 live 93 / 92, 3,803 live 129 / 103.  Nine shape kinds, 65,536
+// slots: 485 live 206 / 453, 2,844 live 700 / 808, 4,009 live 953 / 905; at 8 and 16 steps
+// the lines lie within a quarter of these.
+template <uint32_t kMask> bool serve_by_threads(int64_t nt, int64_t live) {
+  return nav_by_threads<kMask>(NavCall::kTrace, nt) && live >= (kMask == kNavMaskAll ? 3584 : 3072);
+}
+template <uint32_t kMask> void launch_step(vgb_server *s, int64_t nt, int64_t live) {
+  if (serve_by_threads<kMask>(nt, live)) {
     const SrvClient<kMask> c = {s->d_chunks, s->S,       s->pstep,          s->max_steps,
                                 s->steps_per_launch, s->d_live, s->g->dev.nav_flags, s->g->max_depth};
     k_srv_step_tracks<kMask><<<engine_grid(nt), kEngThreads, 0, s->stream>>>(server_geom(s->g), c, nt);
@@ -384,6 +395,7 @@ vgb_status admit(vgb_server *s) {
       }
     }
     std::vector<double>().swap(r->in);
+    r->live = r->n;
     s->active.push_back(r);
   }
   cudaError_t e = cudaMemcpyAsync(s->d_in, s->h_in, 6 * nt * sizeof(double),
@@ -528,9 +540,10 @@ vgb_status vgb_server_step(vgb_server *s, int64_t *completed, int32_t max_comple
   vgb_status st = admit(s);
   if (st != VGB_OK) return st;
   // chunk list of every admitted request
-  int64_t nc = 0;
+  int64_t nc = 0, live_before = 0;
   std::vector<std::pair<int64_t, int64_t>> span(s->active.size());
   for (size_t k = 0; k < s->active.size(); ++k) {
+    live_before += s->active[k]->live;
     span[k].first = nc;
     for (int32_t c : s->active[k]->chunks) s->h_chunks[nc++] = c;
     span[k].second = nc;
@@ -543,9 +556,9 @@ vgb_status vgb_server_step(vgb_server *s, int64_t *completed, int32_t max_comple
     if (e != cudaSuccess) return cuda_error(e, "vgb_server_step: chunk list");
     const int64_t nt = nc * kChunk;
     if (s->all_shapes)
-      launch_step<kNavMaskAll>(s, nt);
+      launch_step<kNavMaskAll>(s, nt, live_before);
     else
-      launch_step<kNavMaskBoxTubeTrd>(s, nt);
+      launch_step<kNavMaskBoxTubeTrd>(s, nt, live_before);
     count_launch();
     e = cudaGetLastError();
     if (e == cudaSuccess)
@@ -562,6 +575,7 @@ vgb_status vgb_server_step(vgb_server *s, int64_t *completed, int32_t max_comple
     for (int64_t c = span[k].first; c < span[k].second; ++c) l += s->h_live[c];
     live_total += l;
     Request *r = s->active[k];
+    r->live = l;
     if (l == 0) {
       fin.push_back(r);
       nf += (int64_t)r->chunks.size();
