@@ -393,15 +393,20 @@ def ref_unplaced(ref: RefLib, spec):
     raise ValueError(k)
 
 
+class Unavailable(NotImplementedError):
+    """A shape that only the reference itself (oracle/_ref, built from its sources) can
+    check, where it is not built."""
+
+
 def oracle_unplaced(orc: Oracle, spec):
-    """Create spec's shape in the C restatement."""
+    """Create spec's shape in the C restatement, which has the box and the tube."""
     p = spec.params
     k = spec.kind
     if k == "box":
         return orc.shape("box", p["dx"], p["dy"], p["dz"])
     if k == "tube":
         return orc.shape("tube", p["rmin"], p["rmax"], p["dz"], p["sphi"], p["dphi"])
-    raise NotImplementedError(k)
+    raise Unavailable(k)
 
 
 def oracle_generic_xform(spec) -> bool:

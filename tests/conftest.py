@@ -32,3 +32,15 @@ def pytest_collection_modifyitems(config, items):
     for it in items:
         if "gpu" in it.keywords:
             it.add_marker(skip)
+
+
+@pytest.hookimpl(wrapper=True)
+def pytest_runtest_call(item):
+    """A test whose oracle is the reference's own build skips where that is not built."""
+    try:
+        return (yield)
+    except NotImplementedError as e:
+        import oracle
+        if isinstance(e, oracle.Unavailable):
+            pytest.skip(f"oracle/_ref not built, and the C restatement has no {e}")
+        raise
