@@ -183,18 +183,24 @@ def pycall():
     return _pycall or None
 
 
-def batch_entries(L):
-    """Addresses of a library's vgb_batch and vgb_batch_device, looked up once per
-    library; None for a handle that lacks either."""
-    e = getattr(L, "_batch_entries", False)
-    if e is False:
+def native_batch(L):
+    """What a batch call through the library handle L needs for the native call: its
+    function and the addresses of L's vgb_batch and vgb_batch_device, looked up once per
+    handle; None where there is none (L lacks an entry, or pycall() is None)."""
+    c = getattr(L, "_native_batch", None)
+    if c is None:
+        m = pycall()
+        if m is None and _pycall is None:
+            return None  # torch may yet be loaded
+        c = ()
         try:
-            e = tuple(ctypes.cast(f, ctypes.c_void_p).value
-                      for f in (L.vgb_batch, L.vgb_batch_device))
+            if m is not None:
+                c = (m.batch, *(ctypes.cast(f, ctypes.c_void_p).value
+                                for f in (L.vgb_batch, L.vgb_batch_device)))
         except (AttributeError, ctypes.ArgumentError):
-            e = None
-        L._batch_entries = e
-    return e
+            pass
+        L._native_batch = c
+    return c or None
 
 
 def check(status: int) -> None:

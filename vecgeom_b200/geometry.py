@@ -136,11 +136,11 @@ class PlacedVolume:
         s = stream.cuda_stream if hasattr(stream, "cuda_stream") else stream
         # plain tensors go through one native call; it leaves everything else, errors
         # included, to the general path below
-        native = L.pycall() if hasattr(points.x, "data_ptr") else None
-        entries = L.batch_entries(g.L) if native is not None else None
-        if entries is not None:
-            st = native.batch(
-                *entries, g.handle.value, self.id, op, points.x, points.y, points.z,
+        native = L.native_batch(g.L) if hasattr(points.x, "data_ptr") else None
+        if native is not None:
+            call, general, device = native
+            st = call(
+                general, device, g.handle.value, self.id, op, points.x, points.y, points.z,
                 dirs.x if dirs is not None else None, dirs.y if dirs is not None else None,
                 dirs.z if dirs is not None else None, step_max, out, aux, daughter, precision, s)
             if st is not None:
