@@ -418,7 +418,9 @@ vgb_status vgb_nav_locate(const vgb_geometry *g, int64_t n, const double *x, con
  * loops (a daughter whose widened box the ray misses or enters beyond the
  * running best step is not evaluated, nor a box daughter whose float safety is
  * certainly above the running minimum; the culling of ABBoxNavigator,
- * navigation/ABBoxNavigator.h:148-452); results equal the FP64 form's. */
+ * navigation/ABBoxNavigator.h:148-452) in calls small enough to give a track a
+ * warp; larger calls (a thread per track) run the FP64 form whatever the
+ * precision.  Results equal the FP64 form's. */
 vgb_status vgb_nav_find_next_boundary_and_step(const vgb_geometry *g, int64_t n, const double *x,
                                                const double *y, const double *z,
                                                const double *dx, const double *dy,
@@ -451,7 +453,8 @@ vgb_status vgb_nav_find_next_boundary_and_step_basket(
  * safeties (at the step's start point).  next_ids, steps and safeties may be
  * NULL; nsteps may not.  A client loop over the reference's calls (which
  * source/benchmarking/NavigationBenchmarker.cpp:48-110 times one step at a time);
- * it has no counterpart of its own in the reference. */
+ * it has no counterpart of its own in the reference.  precision as in
+ * vgb_nav_find_next_boundary_and_step. */
 vgb_status vgb_nav_trace(const vgb_geometry *g, int64_t n, const double *x, const double *y,
                          const double *z, const double *dx, const double *dy, const double *dz,
                          double pstep, int32_t max_steps, int32_t *next_ids, double *steps,
@@ -511,7 +514,10 @@ vgb_status vgb_nav_error_flags(const vgb_geometry *g, uint32_t *flags);
 typedef struct vgb_server vgb_server;
 
 /* max_tracks = 0 sizes the slots to a quarter of the free device memory
- * (at most 2^22 tracks).  Fails with VGB_ENOMEM when the slots do not fit. */
+ * (at most 2^22 tracks).  Fails with VGB_ENOMEM when the slots do not fit.
+ * precision VGB_PREC_FP32_REFINE puts the float screen in front of the daughter
+ * loops of launches that give a track a warp; launches with many live tracks run
+ * the FP64 form whatever the precision.  Results are the same either way. */
 vgb_status vgb_server_create(const vgb_geometry *g, int64_t max_tracks, int32_t steps_per_launch,
                              int32_t max_steps, double pstep, int32_t precision,
                              vgb_server **server);

@@ -14,8 +14,10 @@
 // last class: each is stepped by a whole warp, which searches the daughters' boxes
 // 32 at a time, so no thread holds its block up for a long list; the warps take these
 // tracks one by one as they finish their threads' steps (a fixed share each kept the
-// block waiting: traces of 65,536 detector tracks 3,226 us, now 3,102).  A finished track's slot takes the next track of the block's
-// stream (grid-stride), so blocks stay full while tracks are left.
+// block waiting: traces of 65,536 detector tracks 3,226 us, now 3,102).  A finished
+// track's slot takes the next track of the block's stream (grid-stride): the grid's cap
+// of 1,184 blocks has 151,552 slots, so calls of more tracks than that refill, and in
+// smaller ones a block thins out to its slowest track.
 #pragma once
 #include "navigation.cuh"
 
@@ -185,7 +187,9 @@ VGB_D void nav_engine(const NavGeom &G, const C &client, int64_t n) {
 // daughters' different code one after the other, a class of threads walks one list:
 // steps of 1,024 tracks 63 / 227, of 8,192 347 / 243, of 50,021 3,087 / 493; traces of
 // 16,384 6,315 / 8,258, of 65,536 24,506 / 20,936; ABBox traces of 1,024 1,171 / 6,053,
-// of 16,384 11,199 / 6,964.
+// of 16,384 11,199 / 6,964.  LocatePoint of 12,288 points: detector 14.7 / 16.8, mixed
+// shapes 35.1 / 35.1; of 16,384 17.6 / 18.9 and 43.3 / 35.2; of 24,576 21.9 / 18.8 and
+// 59.6 / 36.6.
 enum class NavCall { kLocate, kStep, kTrace, kAbboxStep, kAbboxTrace };
 template <uint32_t kMask> bool nav_by_threads(NavCall call, int64_t n) {
   const bool mixed = kMask == kNavMaskAll;

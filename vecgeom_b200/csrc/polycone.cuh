@@ -142,7 +142,8 @@ template <class R> struct PolyconeOps {
   // evaluation of one section, so the lanes of a warp evaluate together whatever they
   // skipped.  Bound by the divergence of the cone's DistanceToIn (9 of 32 lanes
   // active); 10 planes, 2^22 mixed points: 582 us with the test's three divisions in
-  // every section's step, 441 with this one.
+  // every section's step, 449 with this one (430 without the divisions of far points;
+  // those behind a call out of line, or made ahead for a bit mask of sections: 560, 444).
   static VGB_HD bool dti_step(const PolyconeP &p, const V3<R> &q, const V3<R> &v, R smax,
                               Walk &w) {
     bool over = false;
