@@ -328,13 +328,25 @@ bool bounded_shape(int type, const double *rec) {
   }
 }
 
+// Whether a shape moves directions as points, itself or in a component.
+bool holds_torus(int type, const double *rec) {
+  if (type != VGB_SHAPE_BOOLEAN) return type == VGB_SHAPE_TORUS;
+  const BooleanP &b = *reinterpret_cast<const BooleanP *>(rec);
+  return b.left.type == VGB_SHAPE_TORUS || b.right.type == VGB_SHAPE_TORUS;
+}
+
 // Whether each placed volume's box may stand for it among its mother's daughters: its
 // shape is bounded and its placement a rigid motion, so that the box can be moved to
-// the mother's frame.
+// the mother's frame.  The FP32+refine form's screen takes the boxes of the other shapes
+// too, but for a torus.
 void mark_bounded(vgb_geometry *g) {
-  std::vector<uint8_t> shape(g->unplaced.size()), rigid(g->raw_xforms.size());
-  for (size_t u = 0; u < shape.size(); ++u)
-    shape[u] = bounded_shape(g->unplaced[u].type, g->params.data() + g->unplaced[u].param_off);
+  std::vector<uint8_t> shape(g->unplaced.size()), screen(g->unplaced.size()),
+      rigid(g->raw_xforms.size());
+  for (size_t u = 0; u < shape.size(); ++u) {
+    const double *rec = g->params.data() + g->unplaced[u].param_off;
+    shape[u] = bounded_shape(g->unplaced[u].type, rec);
+    screen[u] = !holds_torus(g->unplaced[u].type, rec);
+  }
   for (size_t i = 0; i < rigid.size(); ++i) {
     const double *r = g->raw_xforms[i].r;
     bool ok = true;
@@ -345,11 +357,13 @@ void mark_bounded(vgb_geometry *g) {
     rigid[i] = ok;
   }
   g->bounded.resize(g->placed.size());
+  g->screened.resize(g->placed.size());
   for (size_t pv = 0; pv < g->placed.size(); ++pv) {
     const PlacedRec &p = g->placed[pv];
-    bool ok = shape[p.unplaced] && rigid[p.raw_xform] && !(g->xforms[p.xform].flags & kXfQuirk16A);
+    bool ok = rigid[p.raw_xform] && !(g->xforms[p.xform].flags & kXfQuirk16A);
     for (int k = 0; ok && k < 6; ++k) ok = std::fabs(g->pl_box[6 * pv + k]) < 1e30f;
-    g->bounded[pv] = ok;
+    g->bounded[pv] = ok && shape[p.unplaced];
+    g->screened[pv] = ok && screen[p.unplaced];
   }
 }
 
@@ -464,7 +478,8 @@ void build_wide(vgb_geometry *g) {
 __global__ void k_nav_records(const PlacedRec *placed, const UnplacedRec *unplaced,
                               const LogicalRec *logicals, const DXform *xforms,
                               const int32_t *daughters, const float *pl_box,
-                              const uint8_t *bounded, int32_t nplaced, int32_t nslots, NavVol *vols,
+                              const uint8_t *bounded, const uint8_t *screened, int32_t nplaced,
+                              int32_t nslots, NavVol *vols,
                               NavSlot *slots, float4 *slot_box) {
   const int32_t stride = gridDim.x * blockDim.x;
   for (int32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < nplaced; k += stride) {
@@ -478,7 +493,8 @@ __global__ void k_nav_records(const PlacedRec *placed, const UnplacedRec *unplac
     const PlacedRec p = placed[pv];
     const UnplacedRec u = unplaced[p.unplaced];
     slots[k] = NavSlot{xforms[p.xform], u.type, u.param_off, pv, 0};
-    const SlotBox b = slot_box_of(pl_box + 6 * (int64_t)pv, bounded[pv] != 0);
+    SlotBox b = slot_box_of(pl_box + 6 * (int64_t)pv, bounded[pv] != 0);
+    b.lo.w = screened[pv] && !bounded[pv] ? 1.f : 0.f;
     slot_box[2 * k] = b.lo;
     slot_box[2 * k + 1] = b.hi;
   }
@@ -671,7 +687,7 @@ vgb_status vgb_geometry_close(vgb_geometry *g) {
       if (bytes) std::memcpy(host.data() + off, v.data(), bytes);
       return off;
     };
-    const size_t o_bounded = put(g->bounded), o_grids = put(g->grids),
+    const size_t o_bounded = put(g->bounded), o_screened = put(g->screened), o_grids = put(g->grids),
                  o_start = put(g->cell_start), o_items = put(g->cell_items);
     size_t bytes = host.size();
     auto room = [&](size_t n) {
@@ -700,7 +716,8 @@ vgb_status vgb_geometry_close(vgb_geometry *g) {
       const int grid = (int)std::min<size_t>((std::max(np, ns) + 255) / 256, 148 * 8);
       k_nav_records<<<grid, 256>>>(g->dev.placed, g->dev.unplaced, g->dev.logicals, g->dev.xforms,
                                    g->dev.daughters, g->dev.pl_box,
-                                   reinterpret_cast<uint8_t *>(base + o_bounded), (int32_t)np,
+                                   reinterpret_cast<uint8_t *>(base + o_bounded),
+                                   reinterpret_cast<uint8_t *>(base + o_screened), (int32_t)np,
                                    (int32_t)ns, g->dev.vols, g->dev.slots, g->dev.slot_box);
       e = cudaGetLastError();
       if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);

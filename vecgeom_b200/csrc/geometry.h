@@ -106,7 +106,8 @@ struct alignas(16) NavSlot {
 static_assert(sizeof(NavSlot) == 128, "one cache line a slot");
 
 // The box of a daughter as the navigator tests it (lower and upper corner, mother's
-// frame): pl_box, or unbounded where that may not stand for the daughter.
+// frame): pl_box, or unbounded where that may not stand for the daughter (lo.w 1 where
+// the FP32+refine form's screen takes pl_box all the same).
 struct SlotBox {
   float4 lo, hi;
 };
@@ -163,6 +164,7 @@ struct vgb_geometry {
   std::vector<float> ab_box;           // the same boxes rounded to float, as navigated
   std::vector<float4> ab_slot;         // per daughter slot: (lower, 0), (upper, 0)
   std::vector<uint8_t> bounded;        // per placed volume: its box may stand for it
+  std::vector<uint8_t> screened;       // and in the FP32+refine form's screen
   std::vector<vgb::CellGrid> grids;    // cell grids (LogicalRec::grid)
   std::vector<int32_t> cell_start, cell_items;
   bool abbox_ok = true;                // every placed volume's shape has an Extent

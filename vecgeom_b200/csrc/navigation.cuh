@@ -429,51 +429,15 @@ VGB_HD V3<double> nav_inverse_point(const NavXform &X, const V3<double> &l) {
 // ---------------------------------------------------------------------------
 // float screen of the FP32+refine form (ABBoxNavigator's idea, kept exact)
 // ---------------------------------------------------------------------------
-// A daughter's DistanceToIn is only needed when it can beat the running best:
-// a ray that misses the daughter's widened box in the mother's frame, or enters
-// it beyond best, cannot (the box encloses the shape; the widening, 1e-3 mm +
-// 1e-5 of the coordinates, and the relative margin below cover float rounding),
-// so the FP64 call is skipped and the result is unchanged.
-struct RayF {
-  float p[3], inv[3];
-  bool flat[3];
-};
-VGB_HD RayF ray_f(const V3<double> &p, const V3<double> &d) {
-  RayF r;
-  const double pp[3] = {p.x, p.y, p.z}, dd[3] = {d.x, d.y, d.z};
-  for (int k = 0; k < 3; ++k) {
-    r.p[k] = (float)pp[k];
-    r.flat[k] = fabs(dd[k]) < 1e-30;
-    r.inv[k] = r.flat[k] ? 0.f : (float)(1.0 / dd[k]);
-  }
-  return r;
-}
-// true when the box cannot hold a hit closer than `best`
-VGB_HD bool box_skips(const float *b, const RayF &r, double best) {
-  float tn = 0.f, tf = 3.0e38f;
-  for (int k = 0; k < 3; ++k) {
-    if (r.flat[k]) {
-      if (r.p[k] < b[k] || r.p[k] > b[3 + k]) return true;
-      continue;
-    }
-    float t1 = (b[k] - r.p[k]) * r.inv[k], t2 = (b[3 + k] - r.p[k]) * r.inv[k];
-    if (t1 > t2) {
-      const float t = t1;
-      t1 = t2;
-      t2 = t;
-    }
-    tn = tn > t1 ? tn : t1;
-    tf = tf < t2 ? tf : t2;
-  }
-  if (tn > tf * 1.0001f + 1e-4f) return true;  // misses the box
-  const float bf = best < 3.0e38 ? (float)best : 3.0e38f;
-  return tn > bf * 1.0001f + 1e-3f;             // enters it beyond best
-}
+// A daughter's DistanceToIn is only needed when it can beat the running best, which its
+// box decides (wide_meets below), and a box daughter's SafetyToIn when it can be below the
+// running minimum.
 
 // Lower bound of a box daughter's SafetyToIn (BoxImplementation.h:801-818,
 // max_i |l_i| - d_i) in float, minus a margin covering the float rounding of
 // the transform and the subtraction.
 VGB_HD float box_safety_lower(const BoxP &b, const DXform &X, const V3<double> &p) {
+  if (X.flags & kXfQuirk16A) return -3e38f;  // not the motion below
   const float ax = (float)(p.x - X.t[0]), ay = (float)(p.y - X.t[1]), az = (float)(p.z - X.t[2]);
   const bool tr = X.flags & kXfHasTrans;
   const float px = tr ? ax : (float)p.x, py = tr ? ay : (float)p.y, pz = tr ? az : (float)p.z;
@@ -922,10 +886,20 @@ template <class L, uint32_t kMask, bool kScreen = false> struct Navigator {
     R best = step;
     int bi = -1;
     if constexpr (kScreen) {
-      const RayF rf = ray_f(lp, ld);
+      // the boxes by which the FP64 form's warps leave daughters out, and those of the
+      // shapes not argued there; a torus, whose directions move as points, is never left
+      // out
+      const bool boxes = G.slot_box != nullptr;
+      const WidePoint wp = wide_point(lp);
+      const WideLine wl = wide_line(lp, ld);
       for (int d = L::lane(); d < lr.dcount; d += L::N) {
-        if (box_skips(G.pl_box + 6 * (int64_t)nav_placed(G, lr.dfirst + d), rf, best)) continue;
-        const R dd = S::distance_to_in(G, lr.dfirst + d, lp, ld, step);
+        const int32_t k = lr.dfirst + d;
+        if (boxes) {
+          SlotBox b = {G.slot_box[2 * k], G.slot_box[2 * k + 1]};
+          if (b.lo.w != 0.f) b = slot_box_of(G.pl_box + 6 * (int64_t)nav_placed(G, k), true);
+          if (!wide_meets(b.lo, b.hi, wp, wl, best)) continue;
+        }
+        const R dd = S::distance_to_in(G, k, lp, ld, step);
         const bool valid = dd < best && !isinf(dd);
         if (valid) {
           best = dd;
