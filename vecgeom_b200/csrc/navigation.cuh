@@ -510,8 +510,8 @@ VGB_HD bool wide_meets(const float4 &lo4, const float4 &hi4, const WidePoint &t,
   }
   out |= tn - tf > 1e-5f * (fabsf(tn) + fabsf(tf));
   // a negative best bounds nothing: a daughter that the point is in answers -1, however
-  // far behind the point its box begins
-  const float bf = best < 3.0e38 ? fmaxf((float)best, 0.f) : 3.0e38f;
+  // far behind the point its box begins (and nothing improves on a NaN)
+  const float bf = fmaxf((float)best, 0.f);
   out |= tn > bf * 1.0001f + 1e-3f;
   return !out;
 }
@@ -525,8 +525,10 @@ VGB_HD bool wide_near(const float4 &lo, const float4 &hi, const WidePoint &t, do
     const float g = fmaxf(fmaxf(a, b), 0.f);
     d2 += g * g;
   }
-  const float lim = fmaxf((float)best, 0.f) * 1.7323f + 1e-3f;  // sqrt(3) best and a margin
-  return !(d2 > lim * lim) || !(best < 1.0e18);  // (d2 and lim * lim stay in a float's range)
+  // sqrt(3) best and a margin; where lim * lim leaves a float's range everything is near,
+  // and where d2 alone does it is the larger
+  const float lim = fmaxf((float)best, 0.f) * 1.7323f + 1e-3f;
+  return !(d2 > lim * lim);
 }
 
 // The daughters a point may be in: the list of its cell where the volume has a
