@@ -1,6 +1,6 @@
 // cellgrids.cu -- test infrastructure: the sizes of the cell grids that prepare_tables
 // makes over the daughters of wide volumes, beside the searches through them.
-#include "navboxes.cu"
+#include "navboxes.cuh"
 
 // out: daughter slots, grids, entries of the start table, entries of the lists
 extern "C" int cg_sizes(vgb_geometry *g, int64_t *out) {

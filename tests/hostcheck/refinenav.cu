@@ -1,6 +1,6 @@
 // refinenav.cu -- test infrastructure: a step from the world volume by the FP64 and the
 // FP32+refine form of the navigator, with the daughters' boxes, on the host.
-#include "navboxes.cu"
+#include "navboxes.cuh"
 
 template <bool kScreen>
 static void from_world(const NavGeom &G, const V3<double> &p, const V3<double> &d, int32_t &next,

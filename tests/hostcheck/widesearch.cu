@@ -1,6 +1,6 @@
 // widesearch.cu -- test infrastructure: the search of a wide volume's daughters from a
 // given point of the world, with the shape calls it makes counted.
-#include "navboxes.cu"
+#include "navboxes.cuh"
 
 namespace {
 constexpr uint32_t kCounted = kNavMaskAll | (1u << 31);

@@ -1,43 +1,18 @@
 """The cell grids over the daughters of wide volumes: their tables grow with the
 daughters, whatever the daughters' sizes, and searches through them find what the plain
 scan of the daughters finds."""
-import ctypes
-import os
-import subprocess
-
 import numpy as np
 import pytest
 
-from vecgeom_b200 import _lib
+import hostlib
 from vecgeom_b200 import workloads as W
-
-HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(os.path.dirname(HERE), "vecgeom_b200", "csrc")
-OUT = os.path.join(os.path.dirname(HERE), "_build", "hostcheck")
 
 MOST = 32  # cells and list entries a daughter (kCellsPerDaughter)
 
 
 @pytest.fixture(scope="module")
 def cg():
-    so = os.path.join(OUT, "libvgb_cellgrids.so")
-    os.makedirs(OUT, exist_ok=True)
-    srcs = [os.path.join(HERE, "hostcheck", "cellgrids.cu")] + [
-        os.path.join(SRC, f) for f in ("geometry.cu", "unplaced.cu", "geometry_io.cu")]
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-Xcompiler", "-fPIC,-ffp-contract=off",
-                    "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
-                    "-shared", "-o", so, *srcs, "-lcudart"], check=True,
-                   stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
-    L = ctypes.CDLL(so)
-    for name, (res, args) in _lib.SIGNATURES.items():
-        f = getattr(L, name, None)
-        if f is not None:
-            f.restype, f.argtypes = res, args
-    vp = ctypes.c_void_p
-    L.nb_trace.argtypes = ([vp, ctypes.c_int64] + [vp] * 6 + [ctypes.c_int32] * 3 + [vp] * 4)
-    L.cg_sizes.argtypes = [vp, vp]
-    return L
+    return hostlib.navsearch()
 
 
 def build(cg, volumes, daughters, layout):

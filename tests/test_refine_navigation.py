@@ -2,40 +2,16 @@
 shapes whose answers their boxes do not bound (the torus moves directions as points),
 placements that are not rigid motions, hits just behind the point, directions that are
 not unit vectors; in calls of both of the GPU's forms."""
-import ctypes
-import os
-import subprocess
-
 import numpy as np
 import pytest
 
-from vecgeom_b200 import _lib
+import hostlib
 from vecgeom_b200 import workloads as W
-
-HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(os.path.dirname(HERE), "vecgeom_b200", "csrc")
-OUT = os.path.join(os.path.dirname(HERE), "_build", "hostcheck")
 
 
 @pytest.fixture(scope="module")
 def rn():
-    so = os.path.join(OUT, "libvgb_refinenav.so")
-    os.makedirs(OUT, exist_ok=True)
-    srcs = [os.path.join(HERE, "hostcheck", "refinenav.cu")] + [
-        os.path.join(SRC, f) for f in ("geometry.cu", "unplaced.cu", "geometry_io.cu")]
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-Xcompiler", "-fPIC,-ffp-contract=off",
-                    "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
-                    "-shared", "-o", so, *srcs, "-lcudart"], check=True,
-                   stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
-    L = ctypes.CDLL(so)
-    for name, (res, args) in _lib.SIGNATURES.items():
-        f = getattr(L, name, None)
-        if f is not None:
-            f.restype, f.argtypes = res, args
-    vp = ctypes.c_void_p
-    L.rn_from_world.argtypes = [vp, ctypes.c_int64] + [vp] * 6 + [ctypes.c_int32] + [vp] * 3
-    return L
+    return hostlib.navsearch()
 
 
 SPECS = {f"{s.kind}{k}": s for k, s in enumerate(W.zoo_specs() + W.zoo2_specs())}

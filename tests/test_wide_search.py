@@ -1,42 +1,16 @@
 """The search of a wide volume's daughters by a warp (navigation.cuh search_wide).
 CPU, one lane: only the answers asked for are evaluated.  GPU: the queue of a warp, at
 numbers of daughters about multiples of 32, against the host's scan of all of them."""
-import ctypes
-import os
-import subprocess
-
 import numpy as np
 import pytest
 
-from vecgeom_b200 import _lib
+import hostlib
 from vecgeom_b200 import workloads as W
-
-HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(os.path.dirname(HERE), "vecgeom_b200", "csrc")
-OUT = os.path.join(os.path.dirname(HERE), "_build", "hostcheck")
 
 
 @pytest.fixture(scope="module")
 def ws():
-    so = os.path.join(OUT, "libvgb_widesearch.so")
-    os.makedirs(OUT, exist_ok=True)
-    srcs = [os.path.join(HERE, "hostcheck", "widesearch.cu")] + [
-        os.path.join(SRC, f) for f in ("geometry.cu", "unplaced.cu", "geometry_io.cu")]
-    nvcc = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
-    subprocess.run([nvcc, "-std=c++17", "-O2", "-Xcompiler", "-fPIC,-ffp-contract=off",
-                    "--expt-relaxed-constexpr", "-gencode", "arch=compute_100a,code=sm_100a",
-                    "-shared", "-o", so, *srcs, "-lcudart"], check=True,
-                   stdout=subprocess.DEVNULL, stderr=subprocess.DEVNULL)
-    L = ctypes.CDLL(so)
-    for name, (res, args) in _lib.SIGNATURES.items():
-        f = getattr(L, name, None)
-        if f is not None:
-            f.restype, f.argtypes = res, args
-    vp = ctypes.c_void_p
-    L.nb_trace.argtypes = ([vp, ctypes.c_int64] + [vp] * 6 + [ctypes.c_int32] * 3 + [vp] * 4)
-    L.ws_from_world.argtypes = ([vp, ctypes.c_int64] + [vp] * 6 + [ctypes.c_int32] * 2
-                                + [ctypes.c_double] + [vp] * 4)
-    return L
+    return hostlib.navsearch()
 
 
 def build(geometry, specs, count, close):
